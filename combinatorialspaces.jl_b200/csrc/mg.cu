@@ -1642,6 +1642,8 @@ __global__ void __launch_bounds__(256) k_cg_scalar(int phase, int nb, int K, int
   }
 }
 
+#include "mg_tail.cuh"
+
 // ---------------------------------------------------------------------------------------------
 // Hierarchy
 // ---------------------------------------------------------------------------------------------
@@ -1696,8 +1698,26 @@ struct LevelBufs {
   const CT<T>* cs = nullptr;  // per-RHS shifts (coarse_solver 2), K * npanels, shared by all levels
 };
 
+// How a workspace's cycles use the tail kernel (k_tail): levels lt .. last run in one launch on clusters
+// of C CTAs, one per right-hand side.
+struct TailCfg {
+  bool decided = false, on = false;
+  int lt = 0, last = 0, C = 1, pfuse = 0, max_rows = 0;
+  size_t smem = 0;                // dynamic shared memory: the tables, the vectors, the CG sums' block partials
+  uint32_t image_bytes = 0, part = 0, part_len = 0;
+  TailLevel lv[kTailLevels] = {};
+  DArr<unsigned char> image;      // the tables, one image per CTA of a cluster
+};
+struct TailProg {
+  DArr<TailOp> ops;
+  int nops = 0;
+  double bytes = 0.0;  // operator, transfer and dense tables read per launch, and the panels in and out
+};
+
 struct Workspace {
   int K = 0, npanels = 0, prec = 0;
+  TailCfg tail;
+  std::map<int, TailProg> tprog;  // by tail_key(entry, parameter)
   std::vector<LevelBufs<float>> f32;
   std::vector<LevelBufs<double>> f64;
   std::vector<LevelBufs<__half>> f16;  // precision 2: FP16 panels, FP32 arithmetic
@@ -1732,6 +1752,8 @@ struct Workspace {
       if (g) cudaGraphExecDestroy(g);
       g = nullptr;
     }
+    tprog.clear();  // they hold the sweep counts
+    tail = TailCfg();
   }
   ~Workspace() { drop_graphs(); }
 };
@@ -3018,6 +3040,596 @@ static T* smooth_correction(const dec_mg& mg, const Level& L, const Level& Cl, L
   return x;
 }
 
+// ---- the lower levels as one launch (k_tail) -----------------------------------------------------
+// What a tail launch is entered for.
+enum TailEntry {
+  TE_CORRECT = 0,   // b_lt = R r of the level above; cycles with μ = the parameter (and μ - 1, ... 1); z out
+  TE_CYCLE = 1,     // lt = 0: one cycle in place on FP64 panels
+  TE_STEP = 2,      // lt = 0: inner_cycles cycles from zero; the result is stored (0) or added to u (1)
+  TE_FMG = 3,       // full multigrid with `parameter` cycles a level, b restricted from the level above (lt > 0)
+                    // or loaded (lt = 0)
+};
+static int tail_key(int entry, int param) { return entry << 16 | param; }
+
+// Does the level's program use A P (k_sweep_ap's form of the first post-smoothing step)?
+static bool tail_uses_ap(const dec_mg& mg, const Level& L, int l, int pfuse) {
+  const int pre = mg.pre_at(l), post = mg.post_at(l);
+  return mg.opt.smoother == DEC_SMOOTH_CHEBYSHEV && L.ap_ok && post >= 2 && pfuse != 0 &&
+         (pre == 0 || (pfuse == 3 && post == 2));
+}
+
+// The largest coarsest level whose dense product every CTA computes whole (no cluster barrier).
+constexpr int kTailDenseOwn = 100;
+constexpr int kTailRows = 1536;  // rows of a level per CTA
+constexpr int kTailRowsFew = 400;  // where a level has two phases of smoothing or fewer
+// The largest level that every CTA keeps whole: its phase costs one SM's work on all rows instead of a
+// cluster barrier and reads from other CTAs.  The smaller bound where that lets the clusters take one
+// more level.
+constexpr int kTailRep = 700, kTailRepSmall = 256;
+
+// Emits the phases of mu_cycle / cg_mu_cycle / fmg_T, statement for statement.
+struct TailBuilder {
+  const dec_mg& mg;
+  const TailCfg& cfg;
+  std::vector<TailOp> ops;
+
+  bool cg() const { return mg.opt.smoother == DEC_SMOOTH_CG; }
+  TailOp& emit(TailType t, int l) {
+    const TailLevel& L = cfg.lv[l - cfg.lt];
+    TailOp op{};
+    op.type = t;
+    op.level = (uint16_t)(l - cfg.lt);
+    op.n = L.n;
+    op.chunk = L.chunk;
+    op.rep = (uint8_t)L.rep;
+    op.W = (uint16_t)L.W;
+    op.t0 = L.t_col;
+    op.t1 = L.t_off;
+    op.t2 = L.t_diag;
+    op.t3 = L.t_dinv;
+    op.t4 = L.t_pa;
+    op.t5 = L.t_pb;
+    op.b = L.buf[TB_B];
+    ops.push_back(op);
+    return ops.back();
+  }
+  uint32_t buf(int l, int b) const { return cfg.lv[l - cfg.lt].buf[b]; }
+  void interval(const Level& L, double& theta, double& delta, double& sigma) const {
+    const double hi = L.lmax, lo = L.lmax / mg.opt.cheb_ratio;
+    theta = (hi + lo) / 2;
+    delta = (hi - lo) / 2;
+    sigma = theta / delta;
+  }
+  void cheb_n(TailOp& op, int mode, double sigma, double delta, double& rho) const {
+    const double rho_new = 1 / (2 * sigma - rho);
+    op.mode = (uint8_t)mode;
+    op.p0 = rho_new * rho;
+    op.p1 = 2 * rho_new / delta;
+    rho = rho_new;
+  }
+  TailOp& sweep(int l, int x, int b, int out) {
+    TailOp& op = emit(TT_SWEEP, l);
+    op.x = buf(l, x);
+    op.b = buf(l, b);
+    op.out = buf(l, out);
+    return op;
+  }
+  int smooth(int l, int x, bool zero_x, int sweeps) {
+    double theta, delta, sigma;
+    interval(mg.lv[l], theta, delta, sigma);
+    double rho = 1 / sigma;
+    const bool from_zero = zero_x;
+    int other = x == TB_X ? TB_Y : TB_X;
+    for (int it = 0; it < sweeps; ++it) {
+      TailOp& op = sweep(l, x, TB_B, other);
+      if (mg.opt.smoother == DEC_SMOOTH_JACOBI) {
+        op.mode = TM_JACOBI;
+        op.p1 = mg.opt.omega;
+      } else if (it == 0) {
+        op.p1 = 1.0 / theta;
+      } else {
+        cheb_n(op, it == 1 && from_zero ? 0 : TM_PREV, sigma, delta, rho);
+      }
+      if (zero_x) op.mode |= TM_FROM_ZERO;
+      std::swap(x, other);
+      zero_x = false;
+    }
+    return x;
+  }
+  void ap(int l, int b, int out, int z, double theta) {
+    TailOp& op = emit(TT_AP, l);
+    const TailLevel& L = cfg.lv[l - cfg.lt];
+    op.t0 = L.t_apc;
+    op.t1 = L.t_apv;
+    op.b = buf(l, b);
+    op.out = buf(l, out);
+    op.z = buf(l + 1, z);
+    op.p0 = 1.0 / theta;
+  }
+  void restrict_to(int l, int src) {  // the phase's rows are level l + 1's
+    const TailLevel &L = cfg.lv[l - cfg.lt], &Lc = cfg.lv[l + 1 - cfg.lt];
+    TailOp& op = emit(TT_RESTRICT, l);
+    op.n = Lc.n;
+    op.chunk = L.rchunk;
+    op.rep = (uint8_t)(L.rep && Lc.rep);
+    op.split = (uint8_t)(Lc.rep && !L.rep);
+    op.W = (uint16_t)L.Wq;
+    op.t0 = L.t_rself;
+    op.t1 = L.t_ridx;
+    op.t2 = L.t_rw;
+    op.x = buf(l, src);
+    op.out = buf(l + 1, TB_B);
+  }
+  void prolong(int l, int x, int z, bool assign) {
+    TailOp& op = emit(TT_PROLONG, l);
+    op.out = buf(l, x);
+    op.z = buf(l + 1, z);
+    op.add = assign ? 0 : 1;
+  }
+  void zero(int l, int x) { emit(TT_ZERO, l).out = buf(l, x); }
+  void cg_smooth(int l, bool zero_x, int steps) {
+    if (steps == 0) return;
+    TailOp& op = emit(TT_CG, l);
+    op.steps = (uint8_t)steps;
+    op.zero = zero_x ? 1 : 0;
+    op.x = buf(l, TB_X);
+    op.out = buf(l, TB_Y);
+    op.z = buf(l, TB_D);
+    op.t4 = buf(l, TB_P1);
+    op.t5 = buf(l, TB_Q);
+    op.t6 = buf(l, TB_E);
+  }
+  void residual(int l, int x, int out) { sweep(l, x, TB_B, out).mode = TM_RESID; }
+  // the iterate of level l after one μ-cycle from buffer x (zero if zero_x)
+  int cycle(int l, int x, bool zero_x, int mu) {
+    if (cg()) {
+      cg_smooth(l, zero_x, mg.pre_at(l));
+      if (mg.pre_at(l) > 0) zero_x = false;
+      if (l >= cfg.last) {
+        if (zero_x) zero(l, TB_X);
+        return TB_X;
+      }
+      if (!zero_x) residual(l, TB_X, TB_Y);
+      restrict_to(l, zero_x ? TB_B : TB_Y);
+      int z = cycle(l + 1, TB_X, true, mu);
+      if (mu > 1) z = cycle(l + 1, z, false, mu - 1);
+      prolong(l, TB_X, z, zero_x);
+      cg_smooth(l, false, mg.post_at(l));
+      return TB_X;
+    }
+    if (l == mg.lc) {
+      if (mg.opt.coarse_solver == 1) return smooth(l, x, zero_x, std::max(1, mg.pre_at(l) + mg.post_at(l)));
+      TailOp& op = emit(TT_COARSE, l);
+      op.split = cfg.C > 1 && mg.lv[l].n > kTailDenseOwn ? 1 : 0;
+      op.out = buf(l, TB_X);
+      return TB_X;
+    }
+    x = smooth(l, x, zero_x, mg.pre_at(l));
+    zero_x = zero_x && mg.pre_at(l) == 0;
+    int r = TB_B;
+    if (!zero_x) {
+      r = x == TB_X ? TB_Y : TB_X;
+      residual(l, x, r);
+    }
+    restrict_to(l, r);
+    int z = cycle(l + 1, TB_X, true, mu);
+    if (mu > 1) z = cycle(l + 1, z, false, mu - 1);
+    const Level& L = mg.lv[l];
+    const int post = mg.post_at(l);
+    double theta, delta, sigma;
+    interval(L, theta, delta, sigma);
+    double rho = 1 / sigma;
+    if (mg.opt.smoother == DEC_SMOOTH_CHEBYSHEV && post >= 2 && L.ap_ok) {
+      if (zero_x && cfg.pfuse != 0) {  // smooth_prolonged
+        int other = x == TB_X ? TB_Y : TB_X;
+        ap(l, TB_B, other, z, theta);
+        std::swap(x, other);
+        for (int it = 1; it < post; ++it) {
+          TailOp& op = sweep(l, x, TB_B, other);
+          cheb_n(op, it == 1 ? TM_PZ : TM_PREV, sigma, delta, rho);
+          if (it == 1) op.z = buf(l + 1, z);
+          std::swap(x, other);
+        }
+        return x;
+      }
+      if (!zero_x && cfg.pfuse == 3 && post == 2) {  // smooth_correction
+        ap(l, r, TB_D, z, theta);
+        TailOp& op = sweep(l, TB_D, r, x);
+        cheb_n(op, TM_PZ | TM_ADD, sigma, delta, rho);
+        op.z = buf(l + 1, z);
+        return x;
+      }
+    }
+    prolong(l, x, z, zero_x);
+    return smooth(l, x, false, post);
+  }
+  int fmg(int l, int cycles) {
+    int z = TB_X;
+    bool zero = true;
+    if (l < cfg.last) {
+      restrict_to(l, TB_B);
+      const int zc = fmg(l + 1, cycles);
+      prolong(l, z, zc, true);
+      zero = false;
+    }
+    for (int c = 0; c < cycles; ++c) {
+      z = cycle(l, z, zero, mg.opt.mu);
+      zero = false;
+    }
+    if (zero) this->zero(l, z);
+    return z;
+  }
+  void build(int entry, int param) {
+    const int lt = cfg.lt;
+    int z = TB_X;
+    if (lt > 0) {
+      emit(TT_RESTRICT_G, lt).out = buf(lt, TB_B);
+    } else {
+      emit(TT_LOAD, lt).out = buf(lt, TB_B);
+      if (entry == TE_CYCLE) emit(TT_LOADX, lt).out = buf(lt, TB_X);
+    }
+    if (entry == TE_CORRECT) {
+      z = cycle(lt, z, true, param);
+      if (param > 1) z = cycle(lt, z, false, param - 1);
+    } else if (entry == TE_CYCLE) {
+      z = cycle(lt, z, false, mg.opt.mu);
+    } else if (entry == TE_STEP) {
+      for (int c = 0; c < mg.opt.inner_cycles; ++c) z = cycle(lt, z, c == 0, mg.opt.mu);
+    } else {
+      z = fmg(lt, param);
+    }
+    emit(entry == TE_STEP && param ? TT_ADDU : TT_STORE, lt).x = buf(lt, z);
+    if (cfg.C > 1) barriers();
+  }
+  // Which phases start with a cluster barrier.  Rows of a split level are written by their CTA alone and
+  // read by others through `gather`; a level that every CTA keeps is written by each, or pushed to all.
+  // A phase needs the barrier when it reads what others may have written since the last one, writes what
+  // they may still read, follows a push, or pushes (the targets may still be read).
+  void barriers() {
+    bool wrote = true, read = false, pushed = false;  // the first remote access waits for all CTAs to run
+    for (TailOp& op : ops) {
+      const bool split = !cfg.lv[op.level].rep;
+      const bool csplit = op.level + 1 < kTailLevels && cfg.lv[op.level + 1].n > 0 && !cfg.lv[op.level + 1].rep;
+      bool reads = false, writes = false, pushes = false;
+      switch (op.type) {
+        case TT_RESTRICT_G: case TT_LOAD: case TT_LOADX: case TT_ZERO: writes = split; break;
+        case TT_SWEEP:
+          reads = (split && !(op.mode & TM_FROM_ZERO)) || (csplit && (op.mode & TM_PZ));
+          writes = split;
+          break;
+        case TT_AP: case TT_PROLONG: reads = csplit; writes = split; break;
+        case TT_RESTRICT:
+          reads = split;
+          writes = csplit;
+          pushes = split && !csplit;
+          break;
+        case TT_COARSE: pushes = op.split != 0; break;
+        case TT_CG: reads = split && !op.zero; writes = split; break;
+        default: break;  // TT_STORE, TT_ADDU: the CTA's own rows
+      }
+      op.barrier = ((reads && wrote) || (writes && read) || pushed || pushes) ? 1 : 0;
+      if (op.barrier) wrote = read = pushed = false;
+      read |= reads;
+      wrote |= writes;
+      pushed |= pushes;
+      if (op.type == TT_CG && split) {  // its sums' barriers; x += Δx comes after the last
+        read = false;
+        wrote = !op.zero;
+      }
+    }
+  }
+};
+
+// The kernel instances' shared memory and cluster sizes, once per device (not inside a capture); how many
+// clusters of 2, 4, 8 and 16 CTAs the device holds at a time.
+template <class T, bool CL, bool CG>
+static void tail_opt_in_one() {
+  DEC_CUDA(cudaFuncSetAttribute(k_tail<T, CL, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
+  if (CL) DEC_CUDA(cudaFuncSetAttribute(k_tail<T, CL, CG>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+}
+static int tail_clusters(int C) {
+  static std::mutex mu;
+  static bool done[64] = {};
+  static int held[64][kTailMaxCluster + 1] = {};
+  int dev = 0;
+  DEC_CUDA(cudaGetDevice(&dev));
+  require(dev >= 0 && dev < 64, "multigrid: device ordinal out of range");
+  std::lock_guard<std::mutex> lock(mu);
+  if (!done[dev]) {
+    tail_opt_in_one<float, true, false>();
+    tail_opt_in_one<float, false, false>();
+    tail_opt_in_one<double, true, false>();
+    tail_opt_in_one<double, false, false>();
+    tail_opt_in_one<double, true, true>();
+    tail_opt_in_one<double, false, true>();
+    for (int c = 2; c <= kTailMaxCluster; c *= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(c);
+      cfg.blockDim = dim3(kTailThreads);
+      cfg.dynamicSmemBytes = kTailSmem;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = c;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, k_tail<double, true, true>, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n = 0;
+      }
+      held[dev][c] = n;
+    }
+    held[dev][1] = 1 << 20;
+    done[dev] = true;
+  }
+  return held[dev][C];
+}
+
+// The tables and vectors of levels lt .. last at cluster size c.C; false if they do not fit.
+static bool tail_layout(const dec_mg& mg, TailCfg& c, size_t es, int K, int rep_rows) {
+  const bool cg = mg.opt.smoother == DEC_SMOOTH_CG, dense = !cg && mg.opt.coarse_solver != 1;
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 15) / 16 * 16;
+    return (uint32_t)o;
+  };
+  for (auto& l : c.lv) l = TailLevel{};
+  for (int k = c.lt; k <= c.last; ++k) {
+    TailLevel& t = c.lv[k - c.lt];
+    const Level& L = mg.lv[k];
+    t.n = L.n;
+    t.W = L.W;
+    t.Wq = L.Wq;
+    t.rep = c.C == 1 || L.n <= rep_rows;
+    t.chunk = t.rep ? L.n : (L.n + c.C - 1) / c.C;
+    if (cg && !t.rep) t.chunk = (t.chunk + TB / K - 1) / (TB / K) * (TB / K);  // whole blocks of the sums
+    if (t.chunk > c.max_rows) return false;
+  }
+  for (int k = c.lt; k <= c.last; ++k) {
+    TailLevel& t = c.lv[k - c.lt];
+    const Level& L = mg.lv[k];
+    const size_t rows = t.chunk;
+    if (k < c.last || !dense) {
+      t.t_col = take(rows * t.W * 2);
+      t.t_off = take(rows * t.W * es);
+    }
+    t.t_diag = take(rows * es);
+    if (!cg) t.t_dinv = take(rows * es);
+    if (k == c.last) break;
+    const TailLevel& tc = c.lv[k + 1 - c.lt];
+    t.t_pa = take(rows * 2);
+    t.t_pb = take(rows * 2);
+    if (tail_uses_ap(mg, L, k, c.pfuse)) {
+      t.t_apc = take(rows * kApW * 2);
+      t.t_apv = take(rows * kApW * es);
+    }
+    t.rchunk = tc.rep && t.rep ? tc.n : (tc.n + c.C - 1) / c.C;
+    if (!tc.rep) t.rchunk = tc.chunk;
+    t.t_rself = take((size_t)t.rchunk * 2);
+    t.t_ridx = take((size_t)t.rchunk * t.Wq * 2);
+    t.t_rw = take((size_t)t.rchunk * 2 * es);
+  }
+  c.image_bytes = (uint32_t)at;
+  for (int k = c.lt; k <= c.last; ++k) {
+    const int nb = cg ? TB_NBUF
+                   : (mg.opt.smoother == DEC_SMOOTH_CHEBYSHEV && mg.post_at(k) == 2 &&
+                      (mg.pre_at(k) > 0 || mg.opt.mu == 2 || k == 0))
+                       ? 4
+                       : 3;
+    for (int b = 0; b < nb; ++b) c.lv[k - c.lt].buf[b] = take((size_t)c.lv[k - c.lt].chunk * es);
+  }
+  if (cg) {
+    c.part_len = (uint32_t)((c.lv[0].n + TB / K - 1) / (TB / K));
+    c.part = take((size_t)c.part_len * 16);
+  }
+  c.smem = at;
+  return at <= kTailSmem;
+}
+
+// Which levels run in k_tail, and on what clusters: the largest clusters (up to 16 CTAs) of which the
+// device holds one per right-hand side at a time, and from the coarsest level up as many levels as their
+// shared memory takes.  Only while a right-hand side gets a cluster of kTailMinCluster CTAs (7 of 16, or
+// 15 of 8): with more right-hand sides the per-level kernels carry enough rows that a launch is no longer
+// all latency (32 FP32 right-hand sides, four to a cluster: 0.6-0.86 of the per-level kernels' speed).
+// Measured without / with (us): icosphere L6, V(3,3), FP64: 662 / 470 (1 right-hand side), 842 / 644 (8);
+// L4: 435 / 288, 510 / 298; CG V-cycles on L6: 1,292 / 674, W-cycles 4,462 / 1,652.  A V(0,2)-cycle is
+// three phases a level: levels of more than kTailRowsFew rows per CTA stay outside (L6, FP32, 8 right-hand
+// sides: 391 / 378, with L5 inside 395 / 422), and few FP32 right-hand sides altogether (1: 292 / 301;
+// 4: 377 / 351).
+constexpr int kTailMinCluster = 8;
+static void tail_decide(const dec_mg& mg, Workspace& w) {
+  TailCfg& c = w.tail;
+  if (c.decided) return;
+  c = TailCfg();
+  c.decided = true;
+  const dec_mg_options& o = mg.opt;
+  const bool cg = o.smoother == DEC_SMOOTH_CG;
+  if (o.smoother == DEC_SMOOTH_LEARNED || w.prec == 2 || mg.lv.size() < 2 || tune_get("tail", 1) == 0) return;
+  if (!cg && o.coarse_solver == 2) return;  // a shift per right-hand side
+  c.pfuse = tune_get("pfuse", kPfuseDefault);
+  c.last = cg ? (int)mg.lv.size() - 1 : mg.lc;
+  if (c.pfuse == 2 || c.last == 0) return;
+  if (!cg && o.coarse_solver == 0 && mg.lv[c.last].n > kTailRepSmall) return;
+  if (cg && w.K > 8) return;  // blocks of fewer than 32 rows
+  const int groups = w.K * w.npanels;
+  const size_t es = w.prec == 1 ? 4 : 8;
+  for (c.C = kTailMaxCluster; c.C > 1 && tail_clusters(c.C) < groups;) c.C /= 2;
+  if (c.C < kTailMinCluster) return;
+  const int sweeps = mg.pre_at(c.last - 1) + mg.post_at(c.last - 1);
+  const bool few = !cg && o.mu == 1 && sweeps <= 2;
+  if (few && w.prec == 1 && groups < 4) return;
+  c.max_rows = few ? kTailRowsFew : kTailRows;
+  auto fits = [&](int lt, int rep_rows) {
+    c.lt = lt;
+    return c.last - lt < kTailLevels && !mg.lv[lt].gen && tail_layout(mg, c, es, w.K, rep_rows);
+  };
+  auto finest = [&](int rep_rows) {
+    int lt = c.last + 1;
+    while (lt > 0 && fits(lt - 1, rep_rows)) --lt;
+    return lt;
+  };
+  const int lt_small = finest(kTailRepSmall), lt_big = finest(kTailRep);
+  const int rep_rows = lt_small < lt_big ? kTailRepSmall : kTailRep, lt = std::min(lt_small, lt_big);
+  if (lt > c.last || (lt > 0 && mg.lv[lt - 1].gen)) return;
+  if (mg.lv[lt].n <= rep_rows) c.C = 1;  // nothing to split
+  c.on = fits(lt, rep_rows);
+}
+
+static bool stream_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
+// The images of the tail's tables.
+template <class T>
+static void tail_pack(const dec_mg& mg, TailCfg& c) {
+  c.image.alloc((size_t)c.image_bytes * c.C);
+  DEC_CUDA(cudaMemsetAsync(c.image.p, 0, c.image.bytes(), nullptr));
+  const bool dense = mg.opt.smoother != DEC_SMOOTH_CG && mg.opt.coarse_solver != 1;
+  for (int k = c.lt; k <= c.last; ++k) {
+    const Level& L = mg.lv[k];
+    TailPack<T> p = {};
+    p.L = c.lv[k - c.lt];
+    if (k < c.last) p.Lc = c.lv[k + 1 - c.lt];
+    p.C = c.C;
+    p.has_a = k < c.last || !dense;
+    p.has_dinv = mg.opt.smoother != DEC_SMOOTH_CG;
+    p.has_p = p.has_r = k < c.last;
+    p.has_ap = k < c.last && tail_uses_ap(mg, L, k, c.pfuse);
+    p.col = L.col.p;
+    p.pa = L.pa.p;
+    p.pb = L.pb.p;
+    p.apc = L.apc.p;
+    p.rself = L.rself.p;
+    p.ridx = L.ridx.p;
+    p.off = pick<T>(L.off64, L.off32);
+    p.diag = pick<T>(L.diag64, L.diag32);
+    p.dinv = pick<T>(L.dinv64, L.dinv32);
+    p.apv = pick<T>(L.apv64, L.apv32);
+    p.rw = pick<T>(L.rw64, L.rw32);
+    p.image = c.image.p;
+    p.image_bytes = c.image_bytes;
+    k_tail_pack<T><<<dim3(grid_for(std::max(p.L.chunk, p.L.rchunk), 128), c.C), 128>>>(p);
+    DEC_CHECK_LAUNCH();
+  }
+}
+
+// The program of one entry (uploads: before a capture starts).
+static void tail_program(dec_mg& mg, Workspace& w, int entry, int param) {
+  const TailCfg& c = w.tail;
+  if (!c.on || w.tprog.count(tail_key(entry, param))) return;
+  if (!c.image.p) {
+    if (w.prec == 1) tail_pack<float>(mg, w.tail);
+    else tail_pack<double>(mg, w.tail);
+  }
+  TailBuilder b{mg, c, {}};
+  b.build(entry, param);
+  TailProg p;
+  p.ops.upload(b.ops);
+  p.nops = (int)b.ops.size();
+  const double e = w.prec == 1 ? 4.0 : 8.0, kt = (double)w.K * w.npanels;
+  for (const TailOp& op : b.ops) {
+    const Level& L = mg.lv[c.lt + op.level];
+    const double n = L.n;
+    switch (op.type) {
+      case TT_SWEEP: p.bytes += n * (L.W * (4 + e) + 2 * e); break;
+      case TT_AP: p.bytes += n * (kApW * (4 + e) + e); break;
+      case TT_RESTRICT: p.bytes += (double)mg.lv[c.lt + op.level + 1].n * ((L.Wq + 1) * 4.0 + 2 * e); break;
+      case TT_RESTRICT_G: p.bytes += n * ((mg.lv[c.lt - 1].Wq + 1) * 4.0 + 2 * e) + mg.lv[c.lt - 1].n * kt * e; break;
+      case TT_PROLONG: p.bytes += n * 8.0; break;
+      case TT_COARSE: p.bytes += n * n * 8.0; break;
+      case TT_CG: p.bytes += (op.steps + 1) * n * (L.W * (4 + e) + e); break;
+      case TT_LOAD: case TT_LOADX: case TT_STORE: p.bytes += n * kt * e; break;
+      case TT_ADDU: p.bytes += n * kt * 16.0; break;
+      default: break;
+    }
+  }
+  DEC_CUDA(cudaStreamSynchronize(nullptr));  // the tables are read from other streams
+  w.tprog.emplace(tail_key(entry, param), std::move(p));
+}
+
+// Decides the tail and builds the programs of the cycles (host work and uploads: before a capture).
+static void ensure_tail(dec_mg& mg, Workspace& w) {
+  tail_decide(mg, w);
+  if (!w.tail.on) return;
+  if (w.tail.lt > 0) {
+    for (int mu = 1; mu <= mg.opt.mu; ++mu) tail_program(mg, w, TE_CORRECT, mu);
+  } else {
+    if (w.prec == 0) tail_program(mg, w, TE_CYCLE, 0);
+    tail_program(mg, w, TE_STEP, 0);
+    tail_program(mg, w, TE_STEP, 1);
+  }
+}
+
+// Can the tail serve this entry now (decided, covering level 0 or starting below level l, program built)?
+static bool tail_at(const Workspace& w, int l, int entry, int param) {
+  return w.tail.on && w.tail.lt == l && w.tprog.count(tail_key(entry, param)) != 0;
+}
+
+// rf: the residual of level lt - 1 (lt > 0); gb / gx_in / gx: panels of level lt; gu: the FP64 iterate.
+template <class T>
+static void launch_tail(const dec_mg& mg, const Workspace& w, int entry, int param, const T* rf, const T* gb,
+                        const T* gx_in, T* gx, double* gu, cudaStream_t s) {
+  const TailCfg& c = w.tail;
+  const TailProg& prog = w.tprog.at(tail_key(entry, param));
+  TailPrm<T> p = {};
+  p.image = c.image.p;
+  p.image_bytes = c.image_bytes;
+  p.ops = prog.ops.p;
+  p.nops = prog.nops;
+  p.K = w.K;
+  if (c.lt > 0) {
+    const Level& F = mg.lv[c.lt - 1];
+    p.rf = rf;
+    p.rf_stride = (size_t)F.n * w.K;
+    p.g_rself = F.rself.p;
+    p.g_ridx = F.ridx.p;
+    p.g_rw = pick<T>(F.rw64, F.rw32);
+    p.g_Wq = F.Wq;
+  }
+  p.gb = gb;
+  p.gx_in = gx_in;
+  p.gx = gx;
+  p.gu = gu;
+  p.stride = (size_t)mg.lv[c.lt].n * w.K;
+  p.ainv = mg.ainv.p;
+  p.part = c.part;
+  p.part_len = c.part_len;
+  add_bytes(prog.bytes);
+  auto go = [&](auto kern) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(w.K * w.npanels * c.C));
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    int na = 0;
+    if (pdl_enabled()) {
+      at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (c.C > 1) {
+      at[na].id = cudaLaunchAttributeClusterDimension;
+      at[na].val.clusterDim.x = c.C;
+      at[na].val.clusterDim.y = at[na].val.clusterDim.z = 1;
+      ++na;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = na;
+    DEC_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
+  };
+  const bool cg = mg.opt.smoother == DEC_SMOOTH_CG;
+  if constexpr (sizeof(T) == 8) {
+    if (cg) {
+      c.C > 1 ? go(k_tail<double, true, true>) : go(k_tail<double, false, true>);
+      return;
+    }
+  }
+  c.C > 1 ? go(k_tail<T, true, false>) : go(k_tail<T, false, false>);
+}
+
 // steps iterations of the Krylov CG smoother on level L from x (zero if zero_x); returns the
 // buffer holding x.  FP64 only.
 template <int K>
@@ -3086,9 +3698,14 @@ static double* cg_mu_cycle(const dec_mg& mg, Workspace& w, std::vector<LevelBufs
   }
   const Level& Cl = mg.lv[l + 1];
   LevelBufs<double>& Cb = bufs[l + 1];
-  launch_restrict<double, K>(L, Cl, r, Cb.b.p, np, s);
-  double* z = cg_mu_cycle<K>(mg, w, bufs, l + 1, Cb.x.p, true, mu, np, s);
-  if (mu > 1) z = cg_mu_cycle<K>(mg, w, bufs, l + 1, z, false, mu - 1, np, s);
+  double* z = Cb.x.p;
+  if (tail_at(w, l + 1, TE_CORRECT, mu)) {
+    launch_tail<double>(mg, w, TE_CORRECT, mu, r, nullptr, nullptr, z, nullptr, s);
+  } else {
+    launch_restrict<double, K>(L, Cl, r, Cb.b.p, np, s);
+    z = cg_mu_cycle<K>(mg, w, bufs, l + 1, Cb.x.p, true, mu, np, s);
+    if (mu > 1) z = cg_mu_cycle<K>(mg, w, bufs, l + 1, z, false, mu - 1, np, s);
+  }
   launch_prolong<double, K>(L, Cl, (const double*)z, x, zero_x, np, s);
   return cg_smooth<K>(mg, w, L, B, x, false, steps_post, np, s);
 }
@@ -3136,9 +3753,17 @@ static T* mu_cycle(const dec_mg& mg, Workspace& w, std::vector<LevelBufs<T>>& bu
   }
   const Level& Cl = mg.lv[l + 1];
   LevelBufs<T>& Cb = bufs[l + 1];
-  launch_restrict<T, K>(L, Cl, r, Cb.b.p, np, s);
-  T* z = mu_cycle<T, K>(mg, w, bufs, l + 1, Cb.x.p, true, mu, np, s);
-  if (mu > 1) z = mu_cycle<T, K>(mg, w, bufs, l + 1, z, false, mu - 1, np, s);
+  T* z = Cb.x.p;
+  bool in_tail = false;
+  if constexpr (!std::is_same<T, __half>::value) {
+    in_tail = tail_at(w, l + 1, TE_CORRECT, mu);
+    if (in_tail) launch_tail<T>(mg, w, TE_CORRECT, mu, r, nullptr, nullptr, z, nullptr, s);
+  }
+  if (!in_tail) {
+    launch_restrict<T, K>(L, Cl, r, Cb.b.p, np, s);
+    z = mu_cycle<T, K>(mg, w, bufs, l + 1, Cb.x.p, true, mu, np, s);
+    if (mu > 1) z = mu_cycle<T, K>(mg, w, bufs, l + 1, z, false, mu - 1, np, s);
+  }
   if constexpr (!std::is_same<T, __half>::value) {
     if (prolong_fused<T, K>(mg, L, B.cs, mg.post_at(l), zero_x)) {
       if (!zero_x && tune_get("pfuse", kPfuseDefault) == 3)  // r: the restricted residual b - A x
@@ -3243,6 +3868,12 @@ static void enqueue_vcycle_T(dec_mg& mg, Workspace& w, cudaStream_t s, std::vect
   const size_t total = (size_t)mg.lv[0].n * K * w.npanels;
   const int c_last = mg.opt.inner_cycles - 1;
   T* e = bufs[0].x.p;
+  if constexpr (!std::is_same<T, __half>::value) {
+    if (tail_at(w, 0, TE_STEP, upd ? 1 : 0)) {
+      launch_tail<T>(mg, w, TE_STEP, upd ? 1 : 0, nullptr, bufs[0].b.p, nullptr, e, upd, s);
+      return;
+    }
+  }
   for (int c = 0; c <= c_last; ++c)
     e = mu_cycle<T, K>(mg, w, bufs, 0, e, c == 0, mg.opt.mu, w.npanels, s, c == c_last ? upd : nullptr);
   if (!upd && e != bufs[0].x.p) {
@@ -3257,6 +3888,10 @@ template <int K>
 static void enqueue_cycle(dec_mg& mg, Workspace& w, cudaStream_t s) {
   auto& bufs = w.f64;
   const size_t total = (size_t)mg.lv[0].n * K * w.npanels;
+  if (tail_at(w, 0, TE_CYCLE, 0)) {
+    launch_tail<double>(mg, w, TE_CYCLE, 0, nullptr, w.B64.p, w.U64.p, w.U64.p, nullptr, s);
+    return;
+  }
   DEC_CUDA(cudaMemcpyAsync(bufs[0].b.p, w.B64.p, total * sizeof(double), cudaMemcpyDeviceToDevice, s));
   DEC_CUDA(cudaMemcpyAsync(bufs[0].x.p, w.U64.p, total * sizeof(double), cudaMemcpyDeviceToDevice, s));
   double* x = mu_cycle<double, K>(mg, w, bufs, 0, bufs[0].x.p, false, mg.opt.mu, w.npanels, s);
@@ -3351,6 +3986,7 @@ static void ensure_two_step(dec_mg& mg, int K) {
 
 static cudaGraphExec_t capture(dec_mg& mg, Workspace& w, int kind) {
   ensure_two_step(mg, w.K);
+  ensure_tail(mg, w);
   cudaGraph_t g = nullptr;
   require(mg.opt.smoother != DEC_SMOOTH_LEARNED || mg.mlp != nullptr || kind == G_VCYCLE_PLAIN || kind == G_RESID,
           "multigrid: the learned smoother needs a network (dec_mg_set_smoother_mlp)");
@@ -3493,6 +4129,7 @@ static void enqueue_first_rhs(const dec_mg& mg, Workspace& w, cudaStream_t s) {
 // sweep's epilogue (G_STEP) instead of a pass of its own.
 static void capture_solve(dec_mg& mg, Workspace& w, bool zero_guess) {
   ensure_two_step(mg, w.K);
+  ensure_tail(mg, w);
   if (w.bn2.n < (size_t)w.K * w.npanels) w.bn2.alloc((size_t)w.K * w.npanels);
   if (!w.loop.p) w.loop.alloc(1);
   cudaGraph_t g = nullptr;
@@ -3644,8 +4281,13 @@ static T* fmg_T(const dec_mg& mg, Workspace& w, std::vector<LevelBufs<T>>& bufs,
   if (l < last) {
     const Level& Cl = mg.lv[l + 1];
     LevelBufs<T>& Cb = bufs[l + 1];
-    launch_restrict<T, K>(L, Cl, (const T*)B.b.p, Cb.b.p, np, s);
-    T* zc = fmg_T<T, K>(mg, w, bufs, l + 1, cycles, np, s);
+    T* zc = Cb.x.p;
+    if (tail_at(w, l + 1, TE_FMG, cycles)) {
+      launch_tail<T>(mg, w, TE_FMG, cycles, B.b.p, nullptr, nullptr, zc, nullptr, s);
+    } else {
+      launch_restrict<T, K>(L, Cl, (const T*)B.b.p, Cb.b.p, np, s);
+      zc = fmg_T<T, K>(mg, w, bufs, l + 1, cycles, np, s);
+    }
     launch_prolong<T, K>(L, Cl, (const T*)zc, z, true, np, s);
     zero = false;
   }
@@ -3661,6 +4303,10 @@ template <int K>
 static void fmg_K(dec_mg& mg, Workspace& w, int cycles, cudaStream_t s) {
   auto& bufs = w.f64;
   const size_t total = (size_t)mg.lv[0].n * K * w.npanels;
+  if (tail_at(w, 0, TE_FMG, cycles)) {
+    launch_tail<double>(mg, w, TE_FMG, cycles, nullptr, w.B64.p, nullptr, w.U64.p, nullptr, s);
+    return;
+  }
   DEC_CUDA(cudaMemcpyAsync(bufs[0].b.p, w.B64.p, total * sizeof(double), cudaMemcpyDeviceToDevice, s));
   double* z = fmg_T<double, K>(mg, w, bufs, 0, cycles, w.npanels, s);
   DEC_CUDA(cudaMemcpyAsync(w.U64.p, z, total * sizeof(double), cudaMemcpyDeviceToDevice, s));
@@ -3678,6 +4324,11 @@ void mg_full_multigrid(dec_mg* mg, double* u, const double* b, int nrhs, int cyc
   const Level& F = mg->lv[0];
   const int n = F.n;
   const size_t total = (size_t)n * w.K * w.npanels;
+  // the tail's programs are built outside captures; a capture that meets a new `cycles` goes level by level
+  if (cycles < (1 << 16) && !stream_capturing(s)) {
+    ensure_tail(*mg, w);
+    tail_program(*mg, w, TE_FMG, cycles);
+  }
   to_panels(n, nrhs, w.K, w.npanels, F.diperm.p, b, w.B64.p, s);
   DEC_CHECK_LAUNCH();
   switch (w.K) {
@@ -4355,7 +5006,10 @@ static void per_group(dec_batch& bt, F&& f) {
 //   WHILE (test): { per group: V-cycles, u += e, r = b - A u, norms;  test }
 //   per group: u out of panels.
 static cudaGraphExec_t batch_capture(dec_batch& bt, double* const* u, const double* const* rhs, const int* nrhs) {
-  for (size_t q = 0; q < bt.groups.size(); ++q) ensure_two_step(*bt.groups[q], bt.used[q]->K);
+  for (size_t q = 0; q < bt.groups.size(); ++q) {
+    ensure_two_step(*bt.groups[q], bt.used[q]->K);
+    ensure_tail(*bt.groups[q], *bt.used[q]);
+  }
   cudaGraph_t g = nullptr;
   DEC_CUDA(cudaGraphCreate(&g, 0));
   const int G = (int)bt.groups.size();
