@@ -8,6 +8,7 @@
 // without FMA contraction, so results reproduce the reference CPU arithmetic.
 #include <algorithm>
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <type_traits>
 
@@ -469,71 +470,217 @@ static void assemble_geometric_star1(const Mesh& m, bool negate, int& W, DArr<in
 }
 
 // ---- inverse geometric ⋆1: Jacobi-preconditioned BiCGSTAB on A = -⋆1 (FP64) ----------------
-constexpr int kKryBlocks = 256;
-// partial sums of up to three dot products (a_k · b_k) per block, then a fixed-order finish
-__global__ void __launch_bounds__(256) k_kry_dots(int n, int nd, const double* __restrict__ a0,
-                                                  const double* __restrict__ b0, const double* __restrict__ a1,
-                                                  const double* __restrict__ b1, const double* __restrict__ a2,
-                                                  const double* __restrict__ b2, double* __restrict__ partial) {
-  double s0 = 0, s1 = 0, s2 = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    s0 += a0[i] * b0[i];
-    if (nd > 1) s1 += a1[i] * b1[i];
-    if (nd > 2) s2 += a2[i] * b2[i];
-  }
-  __shared__ double sh[3][256];
-  sh[0][threadIdx.x] = s0;
-  sh[1][threadIdx.x] = s1;
-  sh[2][threadIdx.x] = s2;
-  __syncthreads();
-  for (int st = 128; st > 0; st >>= 1) {
-    if (threadIdx.x < st)
-      for (int k = 0; k < 3; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + st];
+//
+// The recurrence runs on the device, one graph with a conditional WHILE node: three kernels a step, each
+// with its dot products finished by the last block to arrive (blocks' sums added in block order), which
+// also takes the step's decisions.  A step's vectors sit in L2 and its time is launches and dependent
+// reductions, so the vector updates are formed inside the products that use them, per neighbour, instead
+// of in passes of their own.  Before, nine kernels and five host read-backs a step: the Lie derivative and
+// dual Laplacian of a 97 x 81 grid (two solves of 6 steps) took 2,350 us.
+struct KryState {
+  double bnorm, rho, rho_old, alpha, omega, beta, best;
+  int it, stall, done, pad;
+  unsigned arrived[4];  // blocks of each kernel that have written their sums
+};
+constexpr int kKryThreads = 256, kKryMaxBlocks = 1184, kKryMaxSteps = 1000;
+
+// Block sums of ND values per thread into partial; in the last block to arrive, the totals in tot (thread
+// 0), summed over the blocks in a fixed order.  Returns true for that thread.
+template <int ND>
+__device__ bool kry_sums(double (&v)[ND], double* partial, unsigned* arrived, double (&tot)[ND]) {
+  __shared__ double sh[ND][kKryThreads / 32];
+  __shared__ bool last;
+  auto block_sum = [&](double (&x)[ND]) {
+#pragma unroll
+    for (int k = 0; k < ND; ++k)
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) x[k] += __shfl_xor_sync(0xffffffffu, x[k], s);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int k = 0; k < ND; ++k) sh[k][threadIdx.x >> 5] = x[k];
     __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int k = 0; k < ND; ++k) {
+        double t = 0.0;
+        for (int w = 0; w < kKryThreads / 32; ++w) t += sh[k][w];
+        x[k] = t;
+      }
+  };
+  block_sum(v);
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < ND; ++k) partial[(size_t)k * kKryMaxBlocks + blockIdx.x] = v[k];
+    __threadfence();
+    last = atomicAdd(arrived, 1u) == gridDim.x - 1;
   }
-  if (threadIdx.x < 3) partial[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = sh[threadIdx.x][0];
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < ND; ++k) {
+    tot[k] = 0.0;
+    for (int b = threadIdx.x; b < gridDim.x; b += kKryThreads)
+      tot[k] += __ldcg(partial + (size_t)k * kKryMaxBlocks + b);
+  }
+  block_sum(tot);
+  if (threadIdx.x != 0) return false;
+  *arrived = 0;
+  return true;
 }
 
-__global__ void k_kry_finish(int nb, const double* __restrict__ partial, double* __restrict__ out) {
-  const int k = threadIdx.x;
-  if (k < 3) {
-    double s = 0;
-    for (int b = 0; b < nb; ++b) s += partial[(size_t)k * nb + b];
-    out[k] = s;
+struct KryVecs {
+  double *b, *x, *r, *rh, *p[2], *v[2], *s, *t, *dinv, *partial;
+};
+
+// b = r = rh = the input, x = p = v = 0, ||b||² (= the first rh·r).
+template <class T>
+__global__ void __launch_bounds__(kKryThreads) k_kry_init(int n, const T* __restrict__ in, KryVecs q, KryState* st) {
+  double s[1] = {0.0}, tot[1];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double v = (double)in[i];
+    q.b[i] = q.r[i] = q.rh[i] = v;
+    q.x[i] = q.p[0][i] = q.v[0][i] = 0.0;
+    s[0] += v * v;
+  }
+  if (kry_sums<1>(s, q.partial, &st->arrived[3], tot)) {
+    st->bnorm = sqrt(tot[0]);
+    st->rho = tot[0];
+    st->rho_old = st->alpha = st->omega = 1.0;
+    st->beta = tot[0];
+    st->best = HUGE_VAL;
+    st->it = st->stall = 0;
+    st->done = (st->bnorm == 0.0 || st->rho == 0.0) ? 1 : 0;
   }
 }
 
-// p = r + β (p - ω v); ph = dinv ∘ p
-__global__ void k_kry_p(int n, double beta, double omega, const double* __restrict__ r, const double* __restrict__ v,
-                        const double* __restrict__ dinv, double* __restrict__ p, double* __restrict__ ph) {
+__global__ void k_kry_start(cudaGraphConditionalHandle h, const KryState* st) {
+  cudaGraphSetConditional(h, st->done ? 0u : 1u);
+}
+
+// p' = r + β (p - ω v), v' = A D⁻¹ p'; rh·v' -> α.  Rows of kGeoWidth slots (slot-major).
+__global__ void __launch_bounds__(kKryThreads) k_kry_v(int n, const int32_t* __restrict__ col,
+                                                       const double* __restrict__ val, KryVecs q, KryState* st) {
+  if (st->done) return;
+  const int o = st->it & 1;
+  const double beta = st->beta, omega = st->omega;
+  const double *r = q.r, *p = q.p[o], *v = q.v[o];
+  double* pn = q.p[1 - o];
+  double* vn = q.v[1 - o];
+  double s[1] = {0.0}, tot[1];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double pi = r[i] + beta * (p[i] - omega * v[i]);
-    p[i] = pi;
-    ph[i] = dinv[i] * pi;
+    double acc = 0.0;
+    int c[kGeoWidth];
+    double a[kGeoWidth];
+#pragma unroll
+    for (int k = 0; k < kGeoWidth; ++k) {
+      c[k] = col[(size_t)k * n + i];
+      a[k] = val[(size_t)k * n + i];
+    }
+#pragma unroll
+    for (int k = 0; k < kGeoWidth; ++k)
+      if (c[k] >= 0) acc += a[k] * (q.dinv[c[k]] * (r[c[k]] + beta * (p[c[k]] - omega * v[c[k]])));
+    pn[i] = r[i] + beta * (p[i] - omega * v[i]);
+    vn[i] = acc;
+    s[0] += q.rh[i] * acc;
+  }
+  if (kry_sums<1>(s, q.partial, &st->arrived[0], tot)) {
+    if (tot[0] == 0.0) st->done = 1;
+    else st->alpha = st->rho / tot[0];
   }
 }
-// s = r - α v; x += α ph; sh = dinv ∘ s
-__global__ void k_kry_s(int n, double alpha, const double* __restrict__ r, const double* __restrict__ v,
-                        const double* __restrict__ ph, const double* __restrict__ dinv, double* __restrict__ s,
-                        double* __restrict__ x, double* __restrict__ shat) {
+
+// s = r - α v', x += α D⁻¹ p', t = A D⁻¹ s; s·s (converged half a step early?), t·s and t·t -> ω.
+__global__ void __launch_bounds__(kKryThreads) k_kry_t(int n, const int32_t* __restrict__ col,
+                                                       const double* __restrict__ val, KryVecs q, KryState* st) {
+  if (st->done) return;
+  const int o = 1 - (st->it & 1);
+  const double alpha = st->alpha;
+  const double *r = q.r, *v = q.v[o], *p = q.p[o];
+  double s[3] = {0.0, 0.0, 0.0}, tot[3];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double acc = 0.0;
+    int c[kGeoWidth];
+    double a[kGeoWidth];
+#pragma unroll
+    for (int k = 0; k < kGeoWidth; ++k) {
+      c[k] = col[(size_t)k * n + i];
+      a[k] = val[(size_t)k * n + i];
+    }
+#pragma unroll
+    for (int k = 0; k < kGeoWidth; ++k)
+      if (c[k] >= 0) acc += a[k] * (q.dinv[c[k]] * (r[c[k]] - alpha * v[c[k]]));
     const double si = r[i] - alpha * v[i];
-    s[i] = si;
-    x[i] += alpha * ph[i];
-    shat[i] = dinv[i] * si;
+    q.x[i] += alpha * (q.dinv[i] * p[i]);
+    q.s[i] = si;
+    q.t[i] = acc;
+    s[0] += si * si;
+    s[1] += acc * si;
+    s[2] += acc * acc;
+  }
+  if (kry_sums<3>(s, q.partial, &st->arrived[1], tot)) {
+    if (sqrt(tot[0]) <= 1e-14 * st->bnorm || tot[2] == 0.0) st->done = 1;
+    else st->omega = tot[1] / tot[2];
   }
 }
-// x += ω sh; r = s - ω t
-__global__ void k_kry_x(int n, double omega, const double* __restrict__ s, const double* __restrict__ t,
-                        const double* __restrict__ shat, double* __restrict__ x, double* __restrict__ r) {
+
+// x += ω D⁻¹ s, r = s - ω t; r·r and rh·r -> stop, or β of the next step; the WHILE node's condition.
+__global__ void __launch_bounds__(kKryThreads) k_kry_r(cudaGraphConditionalHandle h, int n, KryVecs q, KryState* st) {
+  if (st->done) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
+    return;
+  }
+  const double omega = st->omega;
+  double s[2] = {0.0, 0.0}, tot[2];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    x[i] += omega * shat[i];
-    r[i] = s[i] - omega * t[i];
+    const double si = q.s[i];
+    q.x[i] += omega * (q.dinv[i] * si);
+    const double ri = si - omega * q.t[i];
+    q.r[i] = ri;
+    s[0] += ri * ri;
+    s[1] += q.rh[i] * ri;
+  }
+  if (kry_sums<2>(s, q.partial, &st->arrived[2], tot)) {
+    const double rn = sqrt(tot[0]), bn = st->bnorm;
+    bool done = rn <= 1e-14 * bn;
+    if (!done) {
+      if (rn < 0.5 * st->best) {
+        st->best = rn;
+        st->stall = 0;
+      } else if (++st->stall > 20 && rn <= 1e-12 * bn) {
+        done = true;
+      }
+    }
+    const int it = st->it + 1;
+    done = done || omega == 0.0 || tot[1] == 0.0 || !isfinite(rn) || it >= kKryMaxSteps;
+    st->beta = (tot[1] / st->rho) * (st->alpha / omega);
+    st->rho = tot[1];
+    st->it = it;
+    st->done = done ? 1 : 0;
+    cudaGraphSetConditional(h, done ? 0u : 1u);
   }
 }
-__global__ void k_kry_sub(int n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = a[i] - b[i];
+
+// ||b - A x|| and ||b|| into the host's copy.
+__global__ void __launch_bounds__(kKryThreads) k_kry_true(int n, const int32_t* __restrict__ col,
+                                                          const double* __restrict__ val, KryVecs q, KryState* st,
+                                                          double* host) {
+  double s[1] = {0.0}, tot[1];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < kGeoWidth; ++k) {
+      const int c = col[(size_t)k * n + i];
+      if (c >= 0) acc += val[(size_t)k * n + i] * q.x[c];
+    }
+    const double d = q.b[i] - acc;
+    s[0] += d * d;
+  }
+  if (kry_sums<1>(s, q.partial, &st->arrived[3], tot)) {
+    host[0] = sqrt(tot[0]);
+    host[1] = st->bnorm;
+  }
 }
+
 __global__ void k_ell_diag_inv(int n, int W, const int32_t* __restrict__ col, const double* __restrict__ val,
                                double* __restrict__ dinv) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -542,11 +689,6 @@ __global__ void k_ell_diag_inv(int n, int W, const int32_t* __restrict__ col, co
       if (col[(size_t)q * n + i] == i) d += val[(size_t)q * n + i];
     dinv[i] = d != 0.0 ? 1.0 / d : 1.0;
   }
-}
-template <class S, class T>
-__global__ void k_conv(size_t n, const S* __restrict__ a, T* __restrict__ b) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    b[i] = (T)a[i];
 }
 template <class T>
 __global__ void k_epi(size_t n, const double* __restrict__ s, T* __restrict__ y, double alpha, double beta, int hb) {
@@ -683,86 +825,104 @@ static void launch_ell(int n, int W, const int32_t* col, const T* val, const T* 
   else k_ell<T, 0><<<grid_for(n, kOpThreads), kOpThreads, 0, s>>>(n, W, col, val, x, y, a, b, hb);
 }
 
+// What the inverse geometric star keeps with its operator: the vectors, the state, the loop as a graph.
+struct KryPlan {
+  DArr<double> vec;
+  DArr<KryState> state;
+  KryVecs q{};
+  unsigned blocks = 0;
+  cudaGraphExec_t graph = nullptr;
+  double* host = nullptr;  // pinned: true residual norm, ||b||
+  ~KryPlan() {
+    if (graph) cudaGraphExecDestroy(graph);
+    if (host) cudaFreeHost(host);
+  }
+};
+void kry_plan_delete(KryPlan* p) { delete p; }
+
+static KryPlan* kry_plan(const dec_op& op) {
+  const int n = (int)op.rows;
+  const size_t N = ((size_t)n + 31) / 32 * 32;  // every vector aligned
+  auto plan = std::make_unique<KryPlan>();
+  plan->blocks = std::min<unsigned>(kKryMaxBlocks, (unsigned)((n + kKryThreads - 1) / kKryThreads));
+  plan->vec.alloc(11 * N + 3 * kKryMaxBlocks);
+  plan->state.alloc(1);
+  DEC_CUDA(cudaMemset(plan->state.p, 0, sizeof(KryState)));
+  DEC_CUDA(cudaHostAlloc(&plan->host, 2 * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped));
+  double* v = plan->vec.p;
+  KryVecs& q = plan->q;
+  for (double** d : {&q.b, &q.x, &q.r, &q.rh, &q.p[0], &q.p[1], &q.v[0], &q.v[1], &q.s, &q.t, &q.dinv}) {
+    *d = v;
+    v += N;
+  }
+  q.partial = v;
+  k_ell_diag_inv<<<grid_for(n, 256), 256>>>(n, op.W, op.col.p, op.val64.p, q.dinv);
+  DEC_CHECK_LAUNCH();
+  DEC_CUDA(cudaStreamSynchronize(nullptr));
+  cudaStream_t cap;
+  DEC_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+  cudaGraph_t g = nullptr;
+  try {
+    DEC_CUDA(cudaGraphCreate(&g, 0));
+    cudaGraphConditionalHandle h;
+    DEC_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, 0));
+    cudaGraphNode_t start, loop;
+    cudaGraphNodeParams kp = {}, lp = {};
+    KryState* st = plan->state.p;
+    void* args[] = {&h, &st};
+    kp.type = cudaGraphNodeTypeKernel;
+    kp.kernel.func = (void*)k_kry_start;
+    kp.kernel.gridDim = dim3(1);
+    kp.kernel.blockDim = dim3(1);
+    kp.kernel.kernelParams = args;
+    DEC_CUDA(cudaGraphAddNode(&start, g, nullptr, 0, &kp));
+    lp.type = cudaGraphNodeTypeConditional;
+    lp.conditional.handle = h;
+    lp.conditional.type = cudaGraphCondTypeWhile;
+    lp.conditional.size = 1;
+    DEC_CUDA(cudaGraphAddNode(&loop, g, &start, 1, &lp));
+    cudaGraph_t body = lp.conditional.phGraph_out[0];
+    DEC_CUDA(cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    k_kry_v<<<plan->blocks, kKryThreads, 0, cap>>>(n, op.col.p, op.val64.p, q, st);
+    k_kry_t<<<plan->blocks, kKryThreads, 0, cap>>>(n, op.col.p, op.val64.p, q, st);
+    k_kry_r<<<plan->blocks, kKryThreads, 0, cap>>>(h, n, q, st);
+    const cudaError_t err = cudaGetLastError();
+    DEC_CUDA(cudaStreamEndCapture(cap, &body));
+    DEC_CUDA(err);
+    DEC_CUDA(cudaGraphInstantiate(&plan->graph, g, 0));
+  } catch (...) {
+    if (g) cudaGraphDestroy(g);
+    cudaStreamDestroy(cap);
+    throw;
+  }
+  cudaGraphDestroy(g);
+  cudaStreamDestroy(cap);
+  return plan.release();
+}
+
 // y = alpha (-⋆1)⁻¹ x + beta y: BiCGSTAB with the Jacobi preconditioner on A = -⋆1 (stored),
 // FP64, from x0 = 0 to ||b - A x|| <= 1e-14 ||b|| (or 1e-12 once it stagnates).
 static void inverse_geometric_star(dec_op& op, const void* vx, void* vy, double alpha, double beta, cudaStream_t s) {
   const int n = (int)op.rows;
   if (n == 0) return;
+  if (!op.kry) op.kry = kry_plan(op);
+  const KryPlan& k = *op.kry;
   const size_t N = (size_t)n;
-  if (op.kry.n < 10 * N + 4 * kKryBlocks) op.kry.alloc(10 * N + 4 * kKryBlocks);
-  double* b = op.kry.p;
-  double* x = b + N;
-  double* r = x + N;
-  double* rh = r + N;
-  double* p = rh + N;
-  double* v = p + N;
-  double* ph = v + N;
-  double* sv = ph + N;
-  double* t = sv + N;
-  double* dinv = t + N;
-  double* partial = dinv + N;
-  double* dres = partial + 3 * kKryBlocks;
-  const unsigned g = grid_for(n, 256);
-  if (op.dtype == DEC_F64) DEC_CUDA(cudaMemcpyAsync(b, vx, N * 8, cudaMemcpyDeviceToDevice, s));
-  else k_conv<float, double><<<g, 256, 0, s>>>(N, (const float*)vx, b);
-  k_ell_diag_inv<<<g, 256, 0, s>>>(n, op.W, op.col.p, op.val64.p, dinv);
-  DEC_CUDA(cudaMemsetAsync(x, 0, N * 8, s));
-  DEC_CUDA(cudaMemcpyAsync(r, b, N * 8, cudaMemcpyDeviceToDevice, s));
-  DEC_CUDA(cudaMemcpyAsync(rh, b, N * 8, cudaMemcpyDeviceToDevice, s));
-  DEC_CUDA(cudaMemsetAsync(p, 0, N * 8, s));
-  DEC_CUDA(cudaMemsetAsync(v, 0, N * 8, s));
-  double h[3];
-  auto dots = [&](int nd, const double* a0, const double* b0, const double* a1, const double* b1, const double* a2,
-                  const double* b2) {
-    k_kry_dots<<<kKryBlocks, 256, 0, s>>>(n, nd, a0, b0, a1, b1, a2, b2, partial);
-    k_kry_finish<<<1, 32, 0, s>>>(kKryBlocks, partial, dres);
-    DEC_CHECK_LAUNCH();
-    DEC_CUDA(cudaMemcpyAsync(h, dres, sizeof(h), cudaMemcpyDeviceToHost, s));
-    DEC_CUDA(cudaStreamSynchronize(s));
-  };
-  dots(1, b, b, nullptr, nullptr, nullptr, nullptr);
-  const double bnorm = std::sqrt(h[0]);
-  double rho_old = 1, alpha_k = 1, omega = 1, best = HUGE_VAL;
-  int stall = 0;
-  bool done = bnorm == 0.0;
-  for (int it = 0; it < 1000 && !done; ++it) {
-    dots(1, rh, r, nullptr, nullptr, nullptr, nullptr);
-    const double rho = h[0];
-    if (rho == 0.0) break;
-    const double beta_k = (rho / rho_old) * (alpha_k / omega);
-    k_kry_p<<<g, 256, 0, s>>>(n, beta_k, omega, r, v, dinv, p, ph);
-    launch_ell<double>(n, op.W, op.col.p, op.val64.p, ph, v, 1.0, 0.0, false, s);
-    dots(1, rh, v, nullptr, nullptr, nullptr, nullptr);
-    if (h[0] == 0.0) break;
-    alpha_k = rho / h[0];
-    k_kry_s<<<g, 256, 0, s>>>(n, alpha_k, r, v, ph, dinv, sv, x, ph);  // ph now holds dinv ∘ s
-    dots(1, sv, sv, nullptr, nullptr, nullptr, nullptr);
-    if (std::sqrt(h[0]) <= 1e-14 * bnorm) break;
-    launch_ell<double>(n, op.W, op.col.p, op.val64.p, ph, t, 1.0, 0.0, false, s);
-    dots(2, t, sv, t, t, nullptr, nullptr);
-    if (h[1] == 0.0) break;
-    omega = h[0] / h[1];
-    k_kry_x<<<g, 256, 0, s>>>(n, omega, sv, t, ph, x, r);
-    dots(1, r, r, nullptr, nullptr, nullptr, nullptr);
-    const double rn = std::sqrt(h[0]);
-    if (rn <= 1e-14 * bnorm) break;
-    if (rn < 0.5 * best) {
-      best = rn;
-      stall = 0;
-    } else if (++stall > 20 && rn <= 1e-12 * bnorm) {
-      break;
-    }
-    rho_old = rho;
-    if (omega == 0.0) break;
-  }
-  // final check on the true residual
-  launch_ell<double>(n, op.W, op.col.p, op.val64.p, x, t, 1.0, 0.0, false, s);
-  k_kry_sub<<<g, 256, 0, s>>>(n, b, t, r);
-  dots(1, r, r, nullptr, nullptr, nullptr, nullptr);
-  if (!(std::sqrt(h[0]) <= 1e-10 * std::max(bnorm, 1e-300)) && bnorm != 0.0)
+  if (op.dtype == DEC_F64) k_kry_init<<<k.blocks, kKryThreads, 0, s>>>(n, (const double*)vx, k.q, k.state.p);
+  else k_kry_init<<<k.blocks, kKryThreads, 0, s>>>(n, (const float*)vx, k.q, k.state.p);
+  DEC_CHECK_LAUNCH();
+  DEC_CUDA(cudaGraphLaunch(k.graph, s));
+  double* host = nullptr;
+  DEC_CUDA(cudaHostGetDevicePointer(&host, k.host, 0));
+  k_kry_true<<<k.blocks, kKryThreads, 0, s>>>(n, op.col.p, op.val64.p, k.q, k.state.p, host);  // final check
+  DEC_CHECK_LAUNCH();
+  DEC_CUDA(cudaStreamSynchronize(s));
+  const double rn = k.host[0], bnorm = k.host[1];
+  if (!(rn <= 1e-10 * std::max(bnorm, 1e-300)) && bnorm != 0.0)
     throw Error(DEC_ERR_NOT_CONVERGED, "inverse geometric hodge: the Krylov solve did not converge");
-  if (op.dtype == DEC_F64) k_epi<double><<<g, 256, 0, s>>>(N, x, (double*)vy, alpha, beta, beta != 0.0);
-  else k_epi<float><<<g, 256, 0, s>>>(N, x, (float*)vy, alpha, beta, beta != 0.0);
+  const unsigned g = grid_for(n, 256);
+  if (op.dtype == DEC_F64) k_epi<double><<<g, 256, 0, s>>>(N, k.q.x, (double*)vy, alpha, beta, beta != 0.0);
+  else k_epi<float><<<g, 256, 0, s>>>(N, k.q.x, (float*)vy, alpha, beta, beta != 0.0);
   DEC_CHECK_LAUNCH();
 }
 

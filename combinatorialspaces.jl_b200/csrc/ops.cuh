@@ -2,6 +2,11 @@
 #pragma once
 #include "mesh.cuh"
 
+namespace decb {
+struct KryPlan;  // inverse geometric ⋆1: the Krylov vectors, its loop as a graph (ops.cu)
+void kry_plan_delete(KryPlan* p);
+}
+
 struct dec_op {
   decb::Mesh* m = nullptr;
   int kind = 0;
@@ -14,9 +19,14 @@ struct dec_op {
   decb::DArr<int32_t> col;
   decb::DArr<double> val64;
   decb::DArr<float> val32;
-  decb::DArr<double> kry;     // inverse geometric ⋆1: Krylov vectors, 1/diag and reduction scratch
+  decb::KryPlan* kry = nullptr;  // made by the first apply of the inverse geometric ⋆1
   mutable unsigned tuned_at = 0;  // tuning-table version of ell_rows
   mutable int ell_rows = 1;       // rows per thread of the ELL apply (autotuned)
+  dec_op() = default;
+  dec_op(const dec_op&) = delete;
+  ~dec_op() {
+    if (kry) decb::kry_plan_delete(kry);
+  }
 };
 
 namespace decb {
