@@ -23,11 +23,11 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "mlp.cuh"
 #include "ops.cuh"
 
-void op_apply_impl(dec_op* op, const void* x, void* y, double alpha, double beta, void* stream);
 
 namespace decb {
 
@@ -61,8 +61,17 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
 }
 
 __device__ void load_weights(MlpSmem& sm, const MlpWeights& w) {
-  for (int i = threadIdx.x; i < kMlpH * kMlpIn; i += blockDim.x) sm.w1[(i / kMlpIn) * kW1Stride + i % kMlpIn] = w.w1[i];
-  for (int i = threadIdx.x; i < kMlpH * kMlpH; i += blockDim.x) sm.w2[(i / kMlpH) * kW2Stride + i % kMlpH] = w.w2[i];
+  // eight BF16 values per load: a CTA starts with these loads, and element by element they were a chain of
+  // sixteen trips to L2 before its first tile
+  for (int c = threadIdx.x; c < kMlpH * kMlpIn / 8; c += blockDim.x) {
+    const int e = 8 * c;
+    *reinterpret_cast<uint4*>(&sm.w1[(e / kMlpIn) * kW1Stride + e % kMlpIn]) = *reinterpret_cast<const uint4*>(w.w1 + e);
+  }
+#pragma unroll 2
+  for (int c = threadIdx.x; c < kMlpH * kMlpH / 8; c += blockDim.x) {
+    const int e = 8 * c;
+    *reinterpret_cast<uint4*>(&sm.w2[(e / kMlpH) * kW2Stride + e % kMlpH]) = *reinterpret_cast<const uint4*>(w.w2 + e);
+  }
   for (int i = threadIdx.x; i < kMlpH; i += blockDim.x) {
     sm.b1[i] = w.b1[i];
     sm.b2[i] = w.b2[i];
@@ -828,18 +837,31 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
 //   dz1 = dh1 [z1 > 0],
 // and stores the batch columns jbase .. jbase + 31 of the activations x0, h1, relu(z2), dz1, dz2
 // (structure of arrays [row][B], the layout of the gradient contractions) and dy.
+//
+// A warp's tile is one long chain (three rounds of MMAs and the stores), so what counts is how many warps
+// are resident: two CTAs of eight warps per SM (128 registers) run the 2,048 tiles of a 65,536-sample batch
+// in one round, where 169 registers kept one CTA and took two rounds (51 us; 21 with this and the features read back
+// from the forward).
+constexpr int kBwdCtas = 2;
 struct MlpBwdSmem {
   MlpSmem f;                                              // W1, W2, b1, b2, w3, b3
   __align__(16) __nv_bfloat16 w2t[kMlpH * kW2Stride];    // W2ᵀ: row i = column i of W2
 };
 
 __device__ void load_bwd_weights(MlpBwdSmem& sm, const MlpWeights& w) {
-  for (int i = threadIdx.x; i < kMlpH * kMlpH; i += blockDim.x)
-    sm.w2t[(i % kMlpH) * kW2Stride + i / kMlpH] = w.w2[i];  // w2[j][i] -> w2t[i][j]
+#pragma unroll
+  for (int c = 0; c < kMlpH * kMlpH / 8 / kMlpThreads; ++c) {  // w2[j][i] -> w2t[i][j], eight of a row per load
+    const int e = 8 * (c * kMlpThreads + (int)threadIdx.x), j = e / kMlpH, i = e % kMlpH;
+    const uint4 v = *reinterpret_cast<const uint4*>(w.w2 + e);
+    __nv_bfloat16 b[8];
+    memcpy(b, &v, 16);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sm.w2t[(i + k) * kW2Stride + j] = b[k];
+  }
   load_weights(sm.f, w);  // ends with __syncthreads
 }
 
-__device__ __noinline__ void bwd_tile_tc(const MlpBwdSmem& sm, const __nv_bfloat16* xs, float d, float* __restrict__ act,
+__device__ __forceinline__ void bwd_tile_tc(const MlpBwdSmem& sm, const __nv_bfloat16* xs, float d, float* __restrict__ act,
                                             float* __restrict__ dyb, int64_t jbase, int64_t B, int64_t valid) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const uint32_t* X = reinterpret_cast<const uint32_t*>(xs);
@@ -977,7 +999,7 @@ __device__ __noinline__ void bwd_tile_tc(const MlpBwdSmem& sm, const __nv_bfloat
 }
 
 // Backward of n given feature rows with given dL/dy (the gradient check entry point).
-__global__ void __launch_bounds__(kMlpThreads) k_bwd_direct_tc(int64_t n, const float* __restrict__ x,
+__global__ void __launch_bounds__(kMlpThreads, kBwdCtas) k_bwd_direct_tc(int64_t n, const float* __restrict__ x,
                                                                const float* __restrict__ dy, MlpWeights w,
                                                                float* __restrict__ act, float* __restrict__ dyb) {
   __shared__ MlpBwdSmem sm;
@@ -1012,37 +1034,68 @@ __global__ void __launch_bounds__(kMlpThreads) k_bwd_direct_tc(int64_t n, const 
 
 // Features of sample (vertex i, field rs) on a reference-ordered Laplacian / Helmholtz operator of
 // n rows (slot-major ELL, columns sorted, the diagonal inside, padding column -1).
-__device__ void op_features(int i, int n, int Wf, const int32_t* __restrict__ col, const double* __restrict__ val,
-                            const double* __restrict__ rs, float* f, float* dsc) {
+__device__ __forceinline__ void op_features(int i, int n, int Wf, const int32_t* __restrict__ col,
+                                            const double* __restrict__ val, const double* __restrict__ rs, float* f,
+                                            float* dsc) {
   double di = 0.0;
-  for (int q = 0; q < Wf; ++q)
-    if (col[(size_t)q * n + i] == i) di += val[(size_t)q * n + i];
   float nb[6], cp[6], sabs = 0.f;
   int nn = 0;
-  const float dif = (float)di;
-  for (int q = 0; q < Wf; ++q) {
-    const int c = col[(size_t)q * n + i];
-    if (c < 0 || c == i) continue;
-    const float o = (float)val[(size_t)q * n + i];
-    sabs += fabsf(o);
-    if (nn < 6) {
-      nb[nn] = (float)rs[c];
-      cp[nn] = o / dif;
-      ++nn;
+  float dif;
+  if (Wf == 7) {  // a triangle mesh's rows: every load of the row in flight together, no indexed registers
+    int c[7];
+    double v[7];
+    float g[7];
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      c[q] = col[(size_t)q * n + i];
+      v[q] = val[(size_t)q * n + i];
+    }
+#pragma unroll
+    for (int q = 0; q < 7; ++q) g[q] = c[q] >= 0 ? (float)rs[c[q]] : 0.f;
+    int at = 0;  // the diagonal's slot; the columns are sorted, padding comes last
+#pragma unroll
+    for (int q = 0; q < 7; ++q)
+      if (c[q] == i) {
+        di += v[q];
+        at = q;
+      }
+    dif = (float)di;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const bool past = k >= at;
+      const int ck = past ? c[k + 1] : c[k];
+      const float o = (float)(past ? v[k + 1] : v[k]);
+      nb[k] = past ? g[k + 1] : g[k];
+      cp[k] = o / dif;
+      if (ck >= 0) {
+        sabs += fabsf(o);
+        ++nn;
+      }
+    }
+  } else {
+    for (int q = 0; q < Wf; ++q)
+      if (col[(size_t)q * n + i] == i) di += val[(size_t)q * n + i];
+    dif = (float)di;
+    for (int q = 0; q < Wf; ++q) {
+      const int c = col[(size_t)q * n + i];
+      if (c < 0 || c == i) continue;
+      const float o = (float)val[(size_t)q * n + i];
+      sabs += fabsf(o);
+      if (nn < 6) {
+        const float r = (float)rs[c], a = o / dif;
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+          if (k == nn) {
+            nb[k] = r;
+            cp[k] = a;
+          }
+        ++nn;
+      }
     }
   }
   float scale;
   mlp_features((float)rs[i], nb, cp, nn, 1.f - sabs / dif, f, &scale);
   *dsc = scale / dif;
-}
-
-// The features alone, out of line: the backward tile that follows keeps its registers for the MMA
-// fragments.
-__device__ __noinline__ void op_features_only(int i, int n, int Wf, const int32_t* __restrict__ col,
-                                              const double* __restrict__ val, const double* __restrict__ rs,
-                                              float* f) {
-  float dsc;
-  op_features(i, n, Wf, col, val, rs, f, &dsc);
 }
 
 __global__ void k_op_features(int n, int S, int Wf, const int32_t* __restrict__ col, const double* __restrict__ val,
@@ -1058,10 +1111,10 @@ __global__ void k_op_features(int n, int S, int Wf, const int32_t* __restrict__ 
 }
 
 // δ = dscale · MLP(features) for all n·S samples (tensor cores, the inference kernel's numerics).
-__global__ void __launch_bounds__(kMlpThreads) k_train_fwd(int n, int S, int Wf, const int32_t* __restrict__ col,
+__global__ void __launch_bounds__(kMlpThreads, 3) k_train_fwd(int n, int S, int Wf, const int32_t* __restrict__ col,
                                                            const double* __restrict__ val, const double* __restrict__ r,
                                                            MlpWeights w, double* __restrict__ delta,
-                                                           float* __restrict__ dscale) {
+                                                           float* __restrict__ dscale, uint4* __restrict__ feat) {
   __shared__ MlpSmem sm;
   __shared__ __align__(16) __nv_bfloat16 xs[kMlpWarps][kTile * kXsStride];
   load_weights(sm, w);
@@ -1079,6 +1132,11 @@ __global__ void __launch_bounds__(kMlpThreads) k_train_fwd(int n, int S, int Wf,
       for (int k = 0; k < 16; ++k) f[k] = 0.f;
     }
     store_row(xs[warp], lane, f);
+    if (q < N) {  // the BF16 features, which the backward reads back
+      const uint4* row = reinterpret_cast<const uint4*>(xs[warp] + lane * kXsStride);
+      feat[2 * q] = row[0];
+      feat[2 * q + 1] = row[1];
+    }
     __syncwarp();
     const float yv = mlp_tile32(sm, xs[warp]);
     if (q < N) {
@@ -1130,10 +1188,12 @@ static void train_norms(dec_mlp& m, const dec_op* op, const double* r, int S, cu
   DEC_CHECK_LAUNCH();
 }
 
-// dL/dδ = 2 w (A δ - r), w = ⋆0_i / (S n_s); dy = dL/dδ · dscale; loss partials Σ w δ (A δ - 2 r).
+// dL/dδ = 2 w (A δ - r), w = ⋆0_i / (S n_s); dy = dL/dδ · dscale; loss partials Σ w δ (A δ - 2 r).  A δ is
+// formed here row by row (the operator's apply, its products and sums rounded as that kernel's).
 constexpr int kLossBlocks = 512;
-__global__ void __launch_bounds__(256) k_train_loss(int n, int S, const double* __restrict__ r,
-                                                    const double* __restrict__ aq, const double* __restrict__ delta,
+__global__ void __launch_bounds__(256) k_train_loss(int n, int S, int Wf, const int32_t* __restrict__ col,
+                                                    const double* __restrict__ val, const double* __restrict__ r,
+                                                    const double* __restrict__ delta,
                                                     const double* __restrict__ star0, const double* __restrict__ nrm,
                                                     const float* __restrict__ dscale, double* __restrict__ dy,
                                                     double* __restrict__ lpart) {
@@ -1141,9 +1201,16 @@ __global__ void __launch_bounds__(256) k_train_loss(int n, int S, const double* 
   double acc = 0.0;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N; k += (int64_t)gridDim.x * blockDim.x) {
     const int s = (int)(k / n), i = (int)(k % n);
+    const double* ds = delta + (size_t)s * n;
+    double aq = 0.0;
+#pragma unroll 7
+    for (int q = 0; q < Wf; ++q) {
+      const int c = col[(size_t)q * n + i];
+      if (c >= 0) aq = __dadd_rn(aq, __dmul_rn(val[(size_t)q * n + i], ds[c]));
+    }
     const double w = star0[i] / (nrm[s] * S);
-    dy[k] = 2.0 * w * (aq[k] - r[k]) * (double)dscale[k];
-    acc += w * delta[k] * (aq[k] - 2.0 * r[k]);
+    dy[k] = 2.0 * w * (aq - r[k]) * (double)dscale[k];
+    acc += w * delta[k] * (aq - 2.0 * r[k]);
   }
   __shared__ double sh[256];
   sh[threadIdx.x] = acc;
@@ -1164,38 +1231,35 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
 // Backward over the batch: column j is sample j when the fields hold at most B samples, else a
 // sample drawn uniformly with replacement from (seed, step, j); dL/dy is scaled by N / B so the
 // batch gradient estimates the full one.
-__global__ void __launch_bounds__(kMlpThreads) k_train_bwd_tc(int n, int S, int64_t B, uint64_t seed, int64_t step,
-                                                              int Wf, const int32_t* __restrict__ col,
-                                                              const double* __restrict__ val,
-                                                              const double* __restrict__ r, MlpWeights w,
-                                                              const double* __restrict__ dy, float* __restrict__ act,
-                                                              float* __restrict__ dyb) {
+__global__ void __launch_bounds__(kMlpThreads, kBwdCtas) k_train_bwd_tc(int64_t N, int64_t B, uint64_t seed, int64_t step,
+                                                                        const uint4* __restrict__ feat, MlpWeights w,
+                                                                        const double* __restrict__ dy,
+                                                                        float* __restrict__ act, float* __restrict__ dyb) {
   __shared__ MlpBwdSmem sm;
   __shared__ __align__(16) __nv_bfloat16 xs[kMlpWarps][kTile * kXsStride];
   load_bwd_weights(sm, w);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t N = (int64_t)n * S;
   const bool sample = N > B;
   const int64_t Bn = sample ? B : N;
   const double scale = sample ? (double)N / (double)B : 1.0;
   const int64_t ntiles = (Bn + kTile - 1) / kTile;
   for (int64_t tile = (int64_t)blockIdx.x * kMlpWarps + warp; tile < ntiles; tile += (int64_t)gridDim.x * kMlpWarps) {
     const int64_t j = tile * kTile + lane;
-    float f[16], d = 0.f;
+    uint4 f0 = make_uint4(0, 0, 0, 0), f1 = f0;
+    float d = 0.f;
     if (j < Bn) {
       int64_t q = j;
       if (sample) {
         const uint64_t h = mix64(seed + 0x9E3779B97F4A7C15ull * (uint64_t)(step + 1) + 0xD1B54A32D192ED03ull * (uint64_t)j);
         q = (int64_t)(h % (uint64_t)N);
       }
-      const int s = (int)(q / n), i = (int)(q % n);
-      op_features_only(i, n, Wf, col, val, r + (size_t)s * n, f);
+      f0 = feat[2 * q];
+      f1 = feat[2 * q + 1];
       d = (float)(dy[q] * scale);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 16; ++k) f[k] = 0.f;
     }
-    store_row(xs[warp], lane, f);
+    uint4* row = reinterpret_cast<uint4*>(xs[warp] + lane * kXsStride);
+    row[0] = f0;
+    row[1] = f1;
     __syncwarp();
     bwd_tile_tc(sm, xs[warp], d, act, dyb, tile * kTile, Bn, Bn - tile * kTile);
     __syncwarp();
@@ -1204,7 +1268,8 @@ __global__ void __launch_bounds__(kMlpThreads) k_train_bwd_tc(int n, int S, int6
 
 static unsigned bwd_grid(int64_t samples) {
   const long long tiles = (samples + kTile - 1) / kTile;
-  return (unsigned)std::max<long long>(1, std::min<long long>((tiles + kMlpWarps - 1) / kMlpWarps, num_sms() * 4LL));
+  return (unsigned)std::max<long long>(1, std::min<long long>((tiles + kMlpWarps - 1) / kMlpWarps,
+                                                              num_sms() * (long long)kBwdCtas));
 }
 
 // Parameter gradient partials over one chunk of batch columns per CTA, in a fixed order:
@@ -1218,37 +1283,69 @@ constexpr int kGradThreads = 256, kGradChunk = 256, kMaxChunks = 1024;
 // of dz.  A CTA stages 32 samples of every activation row in shared memory at a time; warp w owns
 // the output tiles dW2 rows 16 (w / 2) .. +15, columns 32 (w % 2) .. +31 (four n8 tiles) and dW1
 // rows 16 (w / 2) .., columns 8 (w % 2) .. +7.  db1, db2, dw3 and db3 are sums on the CUDA cores.
-constexpr int kGradStage = 32;
+//
+// What bounds it is bringing the slices in: 1,092 bytes a sample from L2.  They arrive by 16-byte
+// asynchronous copies, the next slice's in flight while this one is multiplied (4-byte copies into one
+// buffer: 53 us for 65,536 samples, now 22).  Rows of 40 floats: the copies stay aligned and the fragments' 8-byte
+// reads of eight rows fall into different banks.
+constexpr int kGradStage = 32, kGradLd = kGradStage + 8, kGradRows = kActRows + 1;  // activation rows, then dy
+constexpr size_t kGradSmem = 2 * sizeof(float) * (size_t)kGradRows * kGradLd;
 
-__global__ void __launch_bounds__(kGradThreads) k_train_grad_tc(int64_t B, int64_t chunk,
+// wide: rows of act and the chunks start on 16-byte boundaries (B and chunk multiples of 4).
+__global__ void __launch_bounds__(kGradThreads) k_train_grad_tc(int64_t B, int64_t chunk, int wide,
                                                                 const float* __restrict__ act,
                                                                 const float* __restrict__ dyb,
                                                                 float* __restrict__ gpart) {
-  // rows of the staged batch slice: the activation rows then dy, kGradStage samples each (+1 pad)
-  constexpr int kRows = kActRows + 1, kLd = kGradStage + 1;
-  __shared__ float sa[kRows * kLd];
+  extern __shared__ __align__(16) float grad_smem[];
+  constexpr int kLd = kGradLd;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int mt = warp >> 1, nh = warp & 1;
   float c2[4][4] = {}, c1[4] = {};
   float sacc = 0.f;  // this thread's bias / w3 sum (threads 0 .. 192)
   const int64_t lo = blockIdx.x * chunk, hi = min(B, lo + chunk);
-  for (int64_t b0 = lo; b0 < hi; b0 += kGradStage) {
-    // the slice arrives by asynchronous copies, all in flight before the one wait (a load and a
-    // store per element serialised the staging on the load latency)
-    for (int e = threadIdx.x; e < kRows * kGradStage; e += kGradThreads) {
-      const int row = e / kGradStage, c = e % kGradStage;
-      const int64_t q = b0 + c;
-      float* dst = sa + row * kLd + c;
-      if (q < hi) {
-        const float* src = row < kActRows ? act + (size_t)row * B + q : dyb + q;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                     "l"(src)
-                     : "memory");
-      } else {
-        *dst = 0.f;
+  auto stage = [&](int64_t b0, float* sa) {
+    if (wide) {
+      constexpr int V = kGradStage / 4;
+      for (int e = threadIdx.x; e < kGradRows * V; e += kGradThreads) {
+        const int row = e / V, c = 4 * (e % V);
+        const int64_t q = b0 + c;
+        float* dst = sa + row * kLd + c;
+        if (q < hi) {  // hi is a multiple of 4 from lo: whole groups
+          const float* src = row < kActRows ? act + (size_t)row * B + q : dyb + q;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                       "l"(src)
+                       : "memory");
+        } else {
+          *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+    } else {
+      for (int e = threadIdx.x; e < kGradRows * kGradStage; e += kGradThreads) {
+        const int row = e / kGradStage, c = e % kGradStage;
+        const int64_t q = b0 + c;
+        float* dst = sa + row * kLd + c;
+        if (q < hi) {
+          const float* src = row < kActRows ? act + (size_t)row * B + q : dyb + q;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                       "l"(src)
+                       : "memory");
+        } else {
+          *dst = 0.f;
+        }
       }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (lo < hi) stage(lo, grad_smem);
+  int buf = 0;
+  for (int64_t b0 = lo; b0 < hi; b0 += kGradStage, buf ^= 1) {
+    const float* sa = grad_smem + buf * kGradRows * kLd;
+    if (b0 + kGradStage < hi) {
+      stage(b0 + kGradStage, grad_smem + (buf ^ 1) * kGradRows * kLd);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
     __syncthreads();
 #pragma unroll
     for (int ks = 0; ks < kGradStage; ks += 16) {
@@ -1256,24 +1353,28 @@ __global__ void __launch_bounds__(kGradThreads) k_train_grad_tc(int64_t B, int64
       auto afrag = [&](int base, uint32_t (&ah)[4], uint32_t (&al)[4]) {
         const float* r0 = sa + (base + 16 * mt + g) * kLd + ks;
         const float* r8 = r0 + 8 * kLd;
-        split_pair(r0[2 * t], r0[2 * t + 1], ah[0], al[0]);
-        split_pair(r8[2 * t], r8[2 * t + 1], ah[1], al[1]);
-        split_pair(r0[2 * t + 8], r0[2 * t + 9], ah[2], al[2]);
-        split_pair(r8[2 * t + 8], r8[2 * t + 9], ah[3], al[3]);
+        auto two = [](const float* q) { return *reinterpret_cast<const float2*>(q); };
+        const float2 a0 = two(r0 + 2 * t), a1 = two(r8 + 2 * t), a2 = two(r0 + 2 * t + 8), a3 = two(r8 + 2 * t + 8);
+        split_pair(a0.x, a0.y, ah[0], al[0]);
+        split_pair(a1.x, a1.y, ah[1], al[1]);
+        split_pair(a2.x, a2.y, ah[2], al[2]);
+        split_pair(a3.x, a3.y, ah[3], al[3]);
       };
       uint32_t ah[4], al[4];
       afrag(kActDz2, ah, al);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const float* h = sa + (kActH1 + 32 * nh + 8 * u + g) * kLd + ks;
-        const uint32_t b0r = pack_bf16(h[2 * t], h[2 * t + 1]), b1r = pack_bf16(h[2 * t + 8], h[2 * t + 9]);
+        const float2 h0 = *reinterpret_cast<const float2*>(h + 2 * t), h1 = *reinterpret_cast<const float2*>(h + 2 * t + 8);
+        const uint32_t b0r = pack_bf16(h0.x, h0.y), b1r = pack_bf16(h1.x, h1.y);
         mma16816(c2[u], ah, b0r, b1r);
         mma16816(c2[u], al, b0r, b1r);
       }
       afrag(kActDz1, ah, al);
       {
         const float* x = sa + (kActX0 + 8 * nh + g) * kLd + ks;
-        const uint32_t b0r = pack_bf16(x[2 * t], x[2 * t + 1]), b1r = pack_bf16(x[2 * t + 8], x[2 * t + 9]);
+        const float2 x0 = *reinterpret_cast<const float2*>(x + 2 * t), x1 = *reinterpret_cast<const float2*>(x + 2 * t + 8);
+        const uint32_t b0r = pack_bf16(x0.x, x0.y), b1r = pack_bf16(x1.x, x1.y);
         mma16816(c1, ah, b0r, b1r);
         mma16816(c1, al, b0r, b1r);
       }
@@ -1287,10 +1388,22 @@ __global__ void __launch_bounds__(kGradThreads) k_train_grad_tc(int64_t B, int64
                                            : sa + kActRows * kLd;
       const float* dy = sa + kActRows * kLd;
       float s = 0.f;
-      if (p >= 2 * kMlpH && p < 3 * kMlpH) {
-        for (int c = 0; c < kGradStage; ++c) s += dy[c] * row[c];
-      } else {
-        for (int c = 0; c < kGradStage; ++c) s += row[c];
+      const bool w3 = p >= 2 * kMlpH && p < 3 * kMlpH;
+#pragma unroll
+      for (int c = 0; c < kGradStage; c += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(row + c);
+        if (w3) {
+          const float4 d = *reinterpret_cast<const float4*>(dy + c);
+          s += d.x * v.x;
+          s += d.y * v.y;
+          s += d.z * v.z;
+          s += d.w * v.w;
+        } else {
+          s += v.x;
+          s += v.y;
+          s += v.z;
+          s += v.w;
+        }
       }
       sacc += s;
     }
@@ -1347,18 +1460,26 @@ __global__ void k_refresh_bf16(const float* __restrict__ p, __nv_bfloat16* __res
   }
 }
 
-// Adam (β1 = 0.9, β2 = 0.999, ε = 1e-8, bias-corrected) on the FP32 masters.
-__global__ void k_adam(int64_t t, float lr, const float* __restrict__ g, float* __restrict__ p, float* __restrict__ m,
-                       float* __restrict__ v) {
+// The gradient from its group sums (k_grad_reduce2's order), then Adam (β1 = 0.9, β2 = 0.999, ε = 1e-8,
+// bias-corrected) on the FP32 masters and the BF16 copies of W1 and W2, in one pass over the parameters.
+__global__ void k_adam(int64_t t, float lr, const float* __restrict__ red, float* __restrict__ g, float* __restrict__ p,
+                       float* __restrict__ m, float* __restrict__ v, __nv_bfloat16* __restrict__ w1b,
+                       __nv_bfloat16* __restrict__ w2b) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpNParam; i += gridDim.x * blockDim.x) {
-    const float gi = g[i];
+    float gi = 0.f;
+#pragma unroll
+    for (int q = 0; q < kReduceGroups; ++q) gi += red[(size_t)q * kMlpNParam + i];
+    g[i] = gi;
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] = pi;
+    if (i < kOffB1) w1b[i - kOffW1] = __float2bfloat16_rn(pi);
+    else if (i >= kOffW2 && i < kOffB2) w2b[i - kOffW2] = __float2bfloat16_rn(pi);
   }
 }
 
@@ -1377,9 +1498,9 @@ static unsigned eval_grid(long long samples) {
 static void ensure_scratch(dec_mlp& m, size_t N, size_t B, int S) {
   if (m.cap_n < N) {
     m.delta.alloc(N);
-    m.q.alloc(N);
     m.dy.alloc(N);
     m.dsc.alloc(N);
+    m.feat.alloc(2 * N);
     m.cap_n = N;
   }
   if (m.cap_b < B) {
@@ -1399,12 +1520,31 @@ static int grad_chunks(int64_t B, int64_t* chunk) {
   return nch;
 }
 
-static void reduce_grad(dec_mlp& m, int64_t B, float* grad, cudaStream_t s) {
+// The batch's gradient as kReduceGroups group sums, returned; the caller adds them.
+static float* grad_groups(dec_mlp& m, int64_t B, cudaStream_t s) {
   int64_t chunk;
   const int nch = grad_chunks(B, &chunk);
-  k_train_grad_tc<<<nch, kGradThreads, 0, s>>>(B, chunk, m.act.p, m.dyb.p, m.gpart.p);
+  static std::mutex mu;
+  static uint64_t done = 0;  // bit per device: the kernel's shared memory above 48 KB
+  int dev = 0;
+  DEC_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= 64 || !(done & (1ull << dev))) {
+      DEC_CUDA(cudaFuncSetAttribute(k_train_grad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem));
+      if (dev < 64) done |= 1ull << dev;
+    }
+  }
+  const int wide = B % 4 == 0 && chunk % 4 == 0;
+  k_train_grad_tc<<<nch, kGradThreads, kGradSmem, s>>>(B, chunk, wide, m.act.p, m.dyb.p, m.gpart.p);
   float* red = m.gpart.p + (size_t)kMaxChunks * kMlpNParam;  // after the chunk partials
   k_grad_reduce<<<dim3((kMlpNParam + 255) / 256, kReduceGroups), 256, 0, s>>>(nch, m.gpart.p, red);
+  DEC_CHECK_LAUNCH();
+  return red;
+}
+
+static void reduce_grad(dec_mlp& m, int64_t B, float* grad, cudaStream_t s) {
+  const float* red = grad_groups(m, B, s);
   k_grad_reduce2<<<(kMlpNParam + 255) / 256, 256, 0, s>>>(red, grad);
   DEC_CHECK_LAUNCH();
 }
@@ -1421,11 +1561,10 @@ static void loss_and_dy(dec_mlp& m, dec_op* op, const double* r, int S, cudaStre
   const int n = op->m->nv;
   const int64_t N = (int64_t)n * S;
   k_train_fwd<<<eval_grid(N), kMlpThreads, 0, s>>>(n, S, op->W, op->col.p, op->val64.p, r, m.view(), m.delta.p,
-                                                   m.dsc.p);
+                                                   m.dsc.p, m.feat.p);
   DEC_CHECK_LAUNCH();
-  for (int j = 0; j < S; ++j) op_apply_impl(op, m.delta.p + (size_t)j * n, m.q.p + (size_t)j * n, 1.0, 0.0, s);
-  k_train_loss<<<kLossBlocks, 256, 0, s>>>(n, S, r, m.q.p, m.delta.p, op->m->star0.p, m.nrm.p, m.dsc.p, m.dy.p,
-                                           m.lpart.p);
+  k_train_loss<<<kLossBlocks, 256, 0, s>>>(n, S, op->W, op->col.p, op->val64.p, r, m.delta.p, op->m->star0.p,
+                                           m.nrm.p, m.dsc.p, m.dy.p, m.lpart.p);
   DEC_CHECK_LAUNCH();
 }
 
@@ -1588,8 +1727,8 @@ void mlp_loss_grad_impl(dec_mlp* m, dec_op* op, const double* r, int S, double* 
   train_norms(*m, op, r, S, s);
   loss_and_dy(*m, op, r, S, s);
   if (grad) {
-    k_train_bwd_tc<<<bwd_grid(N), kMlpThreads, 0, s>>>(n, S, N, 0, 0, op->W, op->col.p, op->val64.p, r,
-                                                         mlp_weights(m), m->dy.p, m->act.p, m->dyb.p);
+    k_train_bwd_tc<<<bwd_grid(N), kMlpThreads, 0, s>>>(N, N, 0, 0, m->feat.p, mlp_weights(m), m->dy.p, m->act.p,
+                                                       m->dyb.p);
     DEC_CHECK_LAUNCH();
     reduce_grad(*m, N, grad, s);
   }
@@ -1608,14 +1747,13 @@ void mlp_train_impl(dec_mlp* m, dec_op* op, const double* r, int S, int steps, d
   train_norms(*m, op, r, S, s);
   for (int it = 0; it < steps; ++it) {
     loss_and_dy(*m, op, r, S, s);
-    k_train_bwd_tc<<<bwd_grid(Bn), kMlpThreads, 0, s>>>(n, S, batch, seed, m->step, op->W, op->col.p, op->val64.p,
-                                                          r, mlp_weights(m), m->dy.p, m->act.p, m->dyb.p);
+    k_train_bwd_tc<<<bwd_grid(Bn), kMlpThreads, 0, s>>>(N, batch, seed, m->step, m->feat.p, mlp_weights(m), m->dy.p,
+                                                        m->act.p, m->dyb.p);
     DEC_CHECK_LAUNCH();
-    reduce_grad(*m, Bn, m->grad.p, s);
+    const float* red = grad_groups(*m, Bn, s);
     ++m->step;
-    k_adam<<<(kMlpNParam + 255) / 256, 256, 0, s>>>(m->step, (float)lr, m->grad.p, m->master.p, m->adam_m.p,
-                                                    m->adam_v.p);
-    k_refresh_bf16<<<16, 256, 0, s>>>(m->master.p, m->w1b.p, m->w2b.p);
+    k_adam<<<(kMlpNParam + 127) / 128, 128, 0, s>>>(m->step, (float)lr, red, m->grad.p, m->master.p, m->adam_m.p,
+                                                    m->adam_v.p, m->w1b.p, m->w2b.p);
     DEC_CHECK_LAUNCH();
     if (losses) losses[it] = host_loss(*m, s);  // the loss before this step's update
   }

@@ -40,7 +40,9 @@ struct MlpWeights {
 __device__ __forceinline__ void mlp_features(float ri, const float* nbr_r, const float* cpl, int nn, float margin,
                                              float* f, float* scale) {
   float s = fabsf(ri);
-  for (int q = 0; q < nn; ++q) s = fmaxf(s, fabsf(nbr_r[q]));
+#pragma unroll
+  for (int q = 0; q < 6; ++q)
+    if (q < nn) s = fmaxf(s, fabsf(nbr_r[q]));
   if (s == 0.0f) s = 1.0f;
   const float inv = 1.0f / s;
   f[0] = ri * inv;
@@ -66,8 +68,9 @@ struct dec_mlp {
   // training scratch (sized on demand)
   size_t cap_n = 0, cap_b = 0;
   decb::DArr<float> act;      // per-sample activations of the backward batch, SoA
-  decb::DArr<double> delta, q, dy;  // per sample: δ, A δ, dL/dy
+  decb::DArr<double> delta, dy;  // per sample: δ, dL/dy
   decb::DArr<float> dsc;            // per sample: s_i / a_ii
+  decb::DArr<uint4> feat;           // per sample: the 16 features in BF16
   decb::DArr<float> dyb;      // dL/dy of the backward batch
   decb::DArr<float> gpart;    // per-chunk gradient partials
   decb::DArr<double> lpart, nrm, npart;
