@@ -1458,9 +1458,12 @@ __global__ void k_split(int n, int Wf, const int32_t* __restrict__ fcol, const d
 // Krylov-CG smoother (the reference's smoother: Krylov.jl cg(A, b, u; itmax = steps) with warm
 // start, atol = rtol = sqrt(eps), called at Multigrid.jl:860 / :871), FP64, one lane per
 // right-hand side.  Every right-hand side j keeps its own scalars in scal[f * ntot + j]:
-enum CgField { CG_GAMMA = 0, CG_PNORM2, CG_EPS, CG_ALPHA, CG_BETA, CG_ACTIVE, CG_UPDP, CG_ITER, CG_NFIELDS };
-// and a kernel sequence per iteration: q = A p (+ p·q partials); reduce + decide α; Δx += α p,
-// r -= α q (+ r·r partials); reduce + decide β; p = r + β p.
+enum CgField { CG_GAMMA = 0, CG_PNORM2, CG_EPS, CG_ALPHA, CG_BETA, CG_ACTIVE, CG_ITER, CG_NFIELDS };
+// and a kernel sequence per iteration: p = r + β p formed inside q = A p (+ p·q partials); sum and decide α;
+// Δx += α p, r -= α q (+ r·r partials); sum and decide β.  Sums are in a fixed order: a block's rows in a
+// tree of halves, then the blocks strided over 256 and in a tree.  (p = r + β p was a pass of its own.  The
+// sums in the last block to arrive instead of a launch of their own measured slower: a V(3,3)-cycle with
+// 32 right-hand sides on icosphere L7 3.4 against 1.4 ms, one block adding 1,184 x 32 partials.)
 
 template <int K>
 __device__ __forceinline__ void block_partials(double v, double* partial) {
@@ -1474,135 +1477,16 @@ __device__ __forceinline__ void block_partials(double v, double* partial) {
   if (threadIdx.x < K) partial[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * K + threadIdx.x] = sh[threadIdx.x];
 }
 
-// r = b - A x0 (x0 = 0 when zero_x), p = r, Δx = 0; partial r·r.
-template <int K, int W>
-__global__ void __launch_bounds__(TB) k_cg_init(int n, int Wr, const int32_t* __restrict__ col,
-                                                const double* __restrict__ off, const double* __restrict__ diag,
-                                                const double* __restrict__ b, const double* __restrict__ x0,
-                                                int zero_x, double* __restrict__ r, double* __restrict__ p,
-                                                double* __restrict__ dx, double* __restrict__ partial, size_t ps) {
-  const int w = W > 0 ? W : Wr;
-  const int k = threadIdx.x % K;
-  const size_t po = (size_t)blockIdx.y * ps + k;
-  double ss = 0.0;
-  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
-    const size_t ik = po + (size_t)i * K;
-    double rv = b[ik];
-    if (!zero_x) {
-      double acc = diag[i] * x0[ik];
-      for (int s = 0; s < w; ++s) acc += off[(size_t)i * w + s] * x0[po + (size_t)col[(size_t)i * w + s] * K];
-      rv = rv - acc;
-    }
-    r[ik] = rv;
-    p[ik] = rv;
-    dx[ik] = 0.0;
-    ss += rv * rv;
-  }
-  block_partials<K>(ss, partial);
-}
-
-// q = A p for active right-hand sides; partial p·q.
-template <int K, int W>
-__global__ void __launch_bounds__(TB) k_cg_spmv(int n, int Wr, const int32_t* __restrict__ col,
-                                                const double* __restrict__ off, const double* __restrict__ diag,
-                                                const double* __restrict__ p, double* __restrict__ q,
-                                                const double* __restrict__ scal, int ntot, double* __restrict__ partial,
-                                                size_t ps) {
-  const int w = W > 0 ? W : Wr;
-  const int k = threadIdx.x % K;
-  const int j = blockIdx.y * K + k;
-  const bool active = scal[CG_ACTIVE * ntot + j] != 0.0;
-  const size_t po = (size_t)blockIdx.y * ps + k;
-  double ss = 0.0;
-  if (active)
-    for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
-      const size_t ik = po + (size_t)i * K;
-      double pi = p[ik];
-      double acc = diag[i] * pi;
-      for (int s = 0; s < w; ++s) acc += off[(size_t)i * w + s] * p[po + (size_t)col[(size_t)i * w + s] * K];
-      q[ik] = acc;
-      ss += pi * acc;
-    }
-  block_partials<K>(ss, partial);
-}
-
-// Δx += α p, r -= α q for active right-hand sides; partial r·r.
-template <int K>
-__global__ void __launch_bounds__(TB) k_cg_axpy(int n, const double* __restrict__ p, const double* __restrict__ q,
-                                                double* __restrict__ dx, double* __restrict__ r,
-                                                const double* __restrict__ scal, int ntot, double* __restrict__ partial,
-                                                size_t ps) {
-  const int k = threadIdx.x % K;
-  const int j = blockIdx.y * K + k;
-  const bool active = scal[CG_ACTIVE * ntot + j] != 0.0;
-  const double a = scal[CG_ALPHA * ntot + j];
-  const size_t po = (size_t)blockIdx.y * ps + k;
-  double ss = 0.0;
-  if (active)
-    for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
-      const size_t ik = po + (size_t)i * K;
-      dx[ik] += a * p[ik];
-      double rv = r[ik] + (-a) * q[ik];
-      r[ik] = rv;
-      ss += rv * rv;
-    }
-  block_partials<K>(ss, partial);
-}
-
-// p = r + β p where the right-hand side continues.
-template <int K>
-__global__ void __launch_bounds__(TB) k_cg_pupd(int n, const double* __restrict__ r, double* __restrict__ p,
-                                                const double* __restrict__ scal, int ntot, size_t ps) {
-  const int k = threadIdx.x % K;
-  const int j = blockIdx.y * K + k;
-  if (scal[CG_UPDP * ntot + j] == 0.0) return;
-  const double bt = scal[CG_BETA * ntot + j];
-  const size_t po = (size_t)blockIdx.y * ps + k;
-  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
-    const size_t ik = po + (size_t)i * K;
-    p[ik] = r[ik] + bt * p[ik];
-  }
-}
-
-// x = Δx + x0 (Krylov adds the warm start back at the end).
-template <int K>
-__global__ void __launch_bounds__(TB) k_cg_finish(int n, const double* __restrict__ x0, int zero_x,
-                                                  const double* __restrict__ dx, double* __restrict__ out, size_t ps) {
-  const int k = threadIdx.x % K;
-  const size_t po = (size_t)blockIdx.y * ps + k;
-  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
-    const size_t ik = po + (size_t)i * K;
-    out[ik] = zero_x ? dx[ik] : dx[ik] + x0[ik];
-  }
-}
-
 enum CgPhase { CG_PH_INIT = 0, CG_PH_ALPHA = 1, CG_PH_BETA = 2 };
 
-// One CTA per right-hand side: sum the block partials (fixed tree order) and take the CG
-// decisions of Krylov.jl's cg for that phase.
-__global__ void __launch_bounds__(256) k_cg_scalar(int phase, int nb, int K, int ntot, int itmax,
-                                                   const double* __restrict__ partial, double* __restrict__ scal) {
-  const int j = blockIdx.x;
-  const int pnl = j / K, k = j % K;
-  double s = 0.0;
-  for (int bq = threadIdx.x; bq < nb; bq += blockDim.x) s += partial[((size_t)pnl * nb + bq) * K + k];
-  __shared__ double sh[256];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int st = 128; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  const double v = sh[0];
+// The decisions of Krylov.jl's cg at a phase, from its sum v, for right-hand side j.
+__device__ inline void cg_decide(int phase, double v, int j, int ntot, int itmax, double* scal) {
   const double eps = 2.220446049250313e-16, rt = 1.4901161193847656e-08;  // eps(Float64), sqrt(eps)
-  double* S = scal;
-  auto F = [&](int f) -> double& { return S[(size_t)f * ntot + j]; };
+  auto F = [&](int f) -> double& { return scal[(size_t)f * ntot + j]; };
   if (phase == CG_PH_INIT) {
     const double gamma = v;
     F(CG_GAMMA) = gamma;
     F(CG_ITER) = 0.0;
-    F(CG_UPDP) = 0.0;
     F(CG_ALPHA) = 0.0;
     if (gamma == 0.0) {  // x0 is a zero-residual solution: return it
       F(CG_ACTIVE) = 0.0;
@@ -1623,7 +1507,6 @@ __global__ void __launch_bounds__(256) k_cg_scalar(int phase, int nb, int K, int
     }
     F(CG_ALPHA) = F(CG_GAMMA) / pAp;
   } else {
-    F(CG_UPDP) = 0.0;
     if (F(CG_ACTIVE) == 0.0) return;
     const double gnext = v;
     const double rnorm = sqrt(gnext);
@@ -1636,9 +1519,148 @@ __global__ void __launch_bounds__(256) k_cg_scalar(int phase, int nb, int K, int
       F(CG_PNORM2) = gnext + beta * beta * F(CG_PNORM2);
       F(CG_GAMMA) = gnext;
     }
-    const bool more = !solved && iter < (double)itmax;
-    F(CG_UPDP) = more ? 1.0 : 0.0;
-    F(CG_ACTIVE) = more ? 1.0 : 0.0;
+    F(CG_ACTIVE) = (!solved && iter < (double)itmax) ? 1.0 : 0.0;
+  }
+}
+
+// One CTA per right-hand side: the sum over the block partials and the decisions of that phase.
+__global__ void __launch_bounds__(256) k_cg_scalar(int phase, int nb, int K, int ntot, int itmax,
+                                                   const double* __restrict__ partial, double* scal) {
+  pdl_enter();
+  const int j = blockIdx.x;
+  const int pnl = j / K, k = j % K;
+  double s = 0.0;
+  for (int bq = threadIdx.x; bq < nb; bq += blockDim.x) s += partial[((size_t)pnl * nb + bq) * K + k];
+  // the tree of halves over 256: across the warps through shared memory, then within one
+  __shared__ double sh[256];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const double* p = sh + threadIdx.x;
+  double t = ((p[0] + p[128]) + (p[64] + p[192])) + ((p[32] + p[160]) + (p[96] + p[224]));
+#pragma unroll
+  for (int st = 16; st > 0; st >>= 1) t += __shfl_xor_sync(0xffffffffu, t, st);
+  if (threadIdx.x == 0) cg_decide(phase, t, j, ntot, itmax, scal);
+}
+
+// a_ii xi + Σ a_ij f(column): rows of six slots round the first off-diagonal product, others the diagonal's
+// (pinned: the tail kernel computes the same bits).
+template <int W, int K, class F>
+__device__ __forceinline__ double cg_row(int i, int Wr, const int32_t* __restrict__ col, const double* __restrict__ off,
+                                         const double* __restrict__ diag, double xi, F f) {
+  if constexpr (W > 0) {
+    int c[W];
+    double v[W], g[W];
+#pragma unroll
+    for (int s = 0; s < W; ++s) {
+      c[s] = col[(size_t)i * W + s];
+      v[s] = off[(size_t)i * W + s];
+    }
+#pragma unroll
+    for (int s = 0; s < W; ++s) g[s] = f(c[s]);
+    double acc = fma_rn(diag[i], xi, mul_rn(v[0], g[0]));
+#pragma unroll
+    for (int s = 1; s < W; ++s) acc = fma_rn(v[s], g[s], acc);
+    return acc;
+  } else {
+    double acc = mul_rn(diag[i], xi);
+    for (int s = 0; s < Wr; ++s) acc = fma_rn(off[(size_t)i * Wr + s], f(col[(size_t)i * Wr + s]), acc);
+    return acc;
+  }
+}
+
+// r = b - A x0 (x0 = 0 when zero_x), Δx = 0; partial r·r.
+template <int K, int W>
+__global__ void __launch_bounds__(TB) k_cg_init(int n, int Wr, const int32_t* __restrict__ col,
+                                                const double* __restrict__ off, const double* __restrict__ diag,
+                                                const double* __restrict__ b, const double* __restrict__ x0,
+                                                int zero_x, double* __restrict__ r, double* __restrict__ dx,
+                                                double* __restrict__ partial, size_t ps) {
+  pdl_enter();
+  const int k = threadIdx.x % K;
+  const size_t po = (size_t)blockIdx.y * ps + k;
+  double ss = 0.0;
+  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
+    const size_t ik = po + (size_t)i * K;
+    double rv = b[ik];
+    if (!zero_x)
+      rv = sub_rn(rv, cg_row<W, K>(i, Wr, col, off, diag, x0[ik], [&](int c) { return x0[po + (size_t)c * K]; }));
+    r[ik] = rv;
+    dx[ik] = 0.0;
+    ss = fma_rn(rv, rv, ss);
+  }
+  block_partials<K>(ss, partial);
+}
+
+// p' = r + β p (p' = r in the first step), q = A p' for active right-hand sides; partial p'·q.  p' goes to a buffer
+// of its own: neighbours still read p.
+template <int K, int W>
+__global__ void __launch_bounds__(TB) k_cg_spmv(int n, int Wr, const int32_t* __restrict__ col,
+                                                const double* __restrict__ off, const double* __restrict__ diag,
+                                                int first, const double* __restrict__ r, const double* __restrict__ p,
+                                                double* __restrict__ pn, double* __restrict__ q,
+                                                const double* __restrict__ scal, int ntot, double* __restrict__ partial,
+                                                size_t ps) {
+  pdl_enter();
+  const int k = threadIdx.x % K;
+  const int j = blockIdx.y * K + k;
+  const bool active = scal[CG_ACTIVE * ntot + j] != 0.0;
+  const double bt = first ? 0.0 : scal[CG_BETA * ntot + j];
+  const size_t po = (size_t)blockIdx.y * ps + k;
+  double ss = 0.0;
+  if (active)
+    for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
+      const size_t ik = po + (size_t)i * K;
+      double pi, acc;
+      if (first) {
+        pi = r[ik];
+        acc = cg_row<W, K>(i, Wr, col, off, diag, pi, [&](int c) { return r[po + (size_t)c * K]; });
+      } else {
+        pi = fma_rn(bt, p[ik], r[ik]);
+        acc = cg_row<W, K>(i, Wr, col, off, diag, pi,
+                           [&](int c) { return fma_rn(bt, p[po + (size_t)c * K], r[po + (size_t)c * K]); });
+      }
+      pn[ik] = pi;
+      q[ik] = acc;
+      ss = fma_rn(pi, acc, ss);
+    }
+  block_partials<K>(ss, partial);
+}
+
+// Δx += α p, r -= α q for active right-hand sides; partial r·r.
+template <int K>
+__global__ void __launch_bounds__(TB) k_cg_axpy(int n, const double* __restrict__ p, const double* __restrict__ q,
+                                                double* __restrict__ dx, double* __restrict__ r,
+                                                const double* __restrict__ scal, int ntot, double* __restrict__ partial,
+                                                size_t ps) {
+  pdl_enter();
+  const int k = threadIdx.x % K;
+  const int j = blockIdx.y * K + k;
+  const bool active = scal[CG_ACTIVE * ntot + j] != 0.0;
+  const double a = scal[CG_ALPHA * ntot + j];
+  const size_t po = (size_t)blockIdx.y * ps + k;
+  double ss = 0.0;
+  if (active)
+    for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
+      const size_t ik = po + (size_t)i * K;
+      dx[ik] = fma_rn(a, p[ik], dx[ik]);
+      const double rv = fma_rn(-a, q[ik], r[ik]);
+      r[ik] = rv;
+      ss = fma_rn(rv, rv, ss);
+    }
+  block_partials<K>(ss, partial);
+}
+
+// x = Δx + x0 (Krylov adds the warm start back at the end).
+template <int K>
+__global__ void __launch_bounds__(TB) k_cg_finish(int n, const double* __restrict__ x0, int zero_x,
+                                                  const double* __restrict__ dx, double* __restrict__ out, size_t ps) {
+  pdl_enter();
+  const int k = threadIdx.x % K;
+  const size_t po = (size_t)blockIdx.y * ps + k;
+  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
+    const size_t ik = po + (size_t)i * K;
+    out[ik] = zero_x ? dx[ik] : dx[ik] + x0[ik];
   }
 }
 
@@ -1694,7 +1716,7 @@ struct Level {
 template <class T>
 struct LevelBufs {
   DArr<T> x, y, b, d;  // x / y ping-pong, b right-hand side, d the learned sweep's residual / CG direction
-  DArr<T> q, e;        // CG smoother: A p and the accumulated correction Δx (CG mode only)
+  DArr<T> q, e, p2;    // CG smoother: A p, the accumulated correction Δx, the second p (CG mode only)
   const CT<T>* cs = nullptr;  // per-RHS shifts (coarse_solver 2), K * npanels, shared by all levels
 };
 
@@ -3639,30 +3661,28 @@ static double* cg_smooth(const dec_mg& mg, Workspace& w, const Level& L, LevelBu
   const int ntot = K * np;
   const size_t ps = (size_t)L.n * K;
   dim3 g(grid_for(L.n, TB / K, 8), np);
-  const int nb = (int)g.x;
   double* r = (x == B.x.p) ? B.y.p : B.x.p;  // r in the free ping-pong buffer
-  double* pp = B.d.p;
-  if (L.W == 6)
-    k_cg_init<K, 6><<<g, TB, 0, s>>>(L.n, L.W, L.col.p, L.off64.p, L.diag64.p, B.b.p, x, zero_x ? 1 : 0, r, pp,
-                                     B.e.p, w.partial.p, ps);
-  else
-    k_cg_init<K, 0><<<g, TB, 0, s>>>(L.n, L.W, L.col.p, L.off64.p, L.diag64.p, B.b.p, x, zero_x ? 1 : 0, r, pp,
-                                     B.e.p, w.partial.p, ps);
-  k_cg_scalar<<<ntot, 256, 0, s>>>(CG_PH_INIT, nb, K, ntot, steps, w.partial.p, w.scal.p);
+  double *p = B.d.p, *pn = B.p2.p;
+  const int32_t* col = L.col.p;
+  const double *off = L.off64.p, *diag = L.diag64.p, *b = B.b.p;
+  double *scal = w.scal.p, *part = w.partial.p;
+  auto decide = [&](int phase) {
+    launch_pdl(k_cg_scalar, dim3(ntot), dim3(256), s, phase, (int)g.x, K, ntot, steps, (const double*)part, scal);
+  };
+  launch_pdl(L.W == 6 ? k_cg_init<K, 6> : k_cg_init<K, 0>, g, dim3(TB), s, L.n, L.W, col, off, diag, b, (const double*)x,
+             zero_x ? 1 : 0, r, B.e.p, part, ps);
+  decide(CG_PH_INIT);
   for (int it = 0; it < steps; ++it) {
-    if (L.W == 6)
-      k_cg_spmv<K, 6><<<g, TB, 0, s>>>(L.n, L.W, L.col.p, L.off64.p, L.diag64.p, pp, B.q.p, w.scal.p, ntot,
-                                       w.partial.p, ps);
-    else
-      k_cg_spmv<K, 0><<<g, TB, 0, s>>>(L.n, L.W, L.col.p, L.off64.p, L.diag64.p, pp, B.q.p, w.scal.p, ntot,
-                                       w.partial.p, ps);
-    k_cg_scalar<<<ntot, 256, 0, s>>>(CG_PH_ALPHA, nb, K, ntot, steps, w.partial.p, w.scal.p);
-    k_cg_axpy<K><<<g, TB, 0, s>>>(L.n, pp, B.q.p, B.e.p, r, w.scal.p, ntot, w.partial.p, ps);
-    k_cg_scalar<<<ntot, 256, 0, s>>>(CG_PH_BETA, nb, K, ntot, steps, w.partial.p, w.scal.p);
-    if (it + 1 < steps) k_cg_pupd<K><<<g, TB, 0, s>>>(L.n, r, pp, w.scal.p, ntot, ps);
+    launch_pdl(L.W == 6 ? k_cg_spmv<K, 6> : k_cg_spmv<K, 0>, g, dim3(TB), s, L.n, L.W, col, off, diag, it == 0 ? 1 : 0,
+               (const double*)r, (const double*)p, pn, B.q.p, (const double*)scal, ntot, part, ps);
+    std::swap(p, pn);
+    decide(CG_PH_ALPHA);
+    launch_pdl(k_cg_axpy<K>, g, dim3(TB), s, L.n, (const double*)p, (const double*)B.q.p, B.e.p, r, (const double*)scal,
+               ntot, part, ps);
+    if (it + 1 < steps) decide(CG_PH_BETA);  // nothing reads the last step's β
   }
   // x + Δx goes into the residual buffer (free again), which becomes the result
-  k_cg_finish<K><<<g, TB, 0, s>>>(L.n, x, zero_x ? 1 : 0, B.e.p, r, ps);
+  launch_pdl(k_cg_finish<K>, g, dim3(TB), s, L.n, (const double*)x, zero_x ? 1 : 0, (const double*)B.e.p, r, ps);
   DEC_CHECK_LAUNCH();
   return r;
 }
@@ -3790,6 +3810,8 @@ static void alloc_bufs(const dec_mg& mg, std::vector<LevelBufs<T>>& bufs, int K,
     if (mg.opt.smoother == DEC_SMOOTH_CG) {
       bufs[l].q.alloc(n);
       bufs[l].e.alloc(n);
+      bufs[l].p2.alloc(n);
+      DEC_CUDA(cudaMemset(bufs[l].p2.p, 0, bufs[l].p2.bytes()));
       DEC_CUDA(cudaMemset(bufs[l].q.p, 0, bufs[l].q.bytes()));
       DEC_CUDA(cudaMemset(bufs[l].e.p, 0, bufs[l].e.bytes()));
     }
