@@ -934,7 +934,11 @@ static void launch_op(const dec_op& op, const void* vx, void* vy, double alpha, 
   const bool hb = beta != 0.0;
   if (op.W == 7 && op.tuned_at != tune_version()) {  // the table changed since the last lookup
     op.tuned_at = tune_version();
-    op.ell_rows = tune_get(ell_key((int)op.rows, op.W, std::is_same<T, float>::value), 1);
+    // FP32 rows, where two per thread still leave every SM its 2,048 threads: two (icosphere L9 Laplacian
+    // 31.1 -> 28.8 us; a 1201 x 999 grid's 16.3 both ways).  FP64 has its bytes in flight with one.
+    const bool f32 = std::is_same<T, float>::value;
+    const int rows = f32 && op.rows >= 2LL * 2048 * num_sms() ? 2 : 1;
+    op.ell_rows = tune_get(ell_key((int)op.rows, op.W, f32), rows);
   }
   if (op.kind == DEC_OP_GENERAL) {  // a caller's matrix: no mesh
     const T* val = std::is_same<T, double>::value ? (const T*)op.val64.p : (const T*)op.val32.p;

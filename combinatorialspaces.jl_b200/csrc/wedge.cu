@@ -226,6 +226,37 @@ __global__ void __launch_bounds__(kThreads) k_w01v64(int ne, const int32_t* __re
     out[e] = half * a[e] * (__ldg(f + ev0[e]) + __ldg(f + ev1[e]));
 }
 
+// FP64 ∧02 with two consecutive triangles per thread: 8-byte index loads, 16-byte coefficient and form loads
+// and stores, both triangles' gathers in flight; the expression unchanged.  Bound by its bytes (72 a triangle):
+// icosphere L9 49.8 -> 41.4 us, a 1201 x 999 grid 20.8 -> 18.6, L8 14.7 -> 12.5.  (The same for ∧11 measured
+// slower, 67.8 -> 71.2 us on L9: twelve gathers a thread, so it keeps its own kernel.)
+__device__ __forceinline__ double2 ldcs2(const double* p, int g) { return __ldcs(reinterpret_cast<const double2*>(p) + g); }
+__device__ __forceinline__ int2 ldcs2(const int32_t* p, int g) { return __ldcs(reinterpret_cast<const int2*>(p) + g); }
+
+__global__ void __launch_bounds__(kThreads) k_w02v64(int nt, const int32_t* __restrict__ tv0,
+                                                     const int32_t* __restrict__ tv1, const int32_t* __restrict__ tv2,
+                                                     const double* __restrict__ w0, const double* __restrict__ w1,
+                                                     const double* __restrict__ w2, const double* __restrict__ f,
+                                                     const double* __restrict__ a, double* __restrict__ out, size_t sf,
+                                                     size_t sa, size_t so) {
+  f += blockIdx.y * sf;
+  a += blockIdx.y * sa;
+  out += blockIdx.y * so;
+  const int n2 = nt / 2;
+  for (int g = blockIdx.x * kThreads + threadIdx.x; g < n2; g += gridDim.x * kThreads) {
+    const int2 p = ldcs2(tv0, g), q = ldcs2(tv1, g), r = ldcs2(tv2, g);
+    const double2 c0 = ldcs2(w0, g), c1 = ldcs2(w1, g), c2 = ldcs2(w2, g), av = ldcs2(a, g);
+    const double x0 = __ldg(f + p.x), x1 = __ldg(f + q.x), x2 = __ldg(f + r.x);
+    const double y0 = __ldg(f + p.y), y1 = __ldg(f + q.y), y2 = __ldg(f + r.y);
+    __stcs(reinterpret_cast<double2*>(out) + g,
+           make_double2(av.x * (c0.x * x0 + c1.x * x1 + c2.x * x2), av.y * (c0.y * y0 + c1.y * y1 + c2.y * y2)));
+  }
+  if ((nt & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+    const int t = nt - 1;
+    out[t] = a[t] * (w0[t] * f[tv0[t]] + w1[t] * f[tv1[t]] + w2[t] * f[tv2[t]]);
+  }
+}
+
 __global__ void __launch_bounds__(kThreads) k_w02v(int nt, const int32_t* __restrict__ tv0,
                                                    const int32_t* __restrict__ tv1, const int32_t* __restrict__ tv2,
                                                    const float* __restrict__ w0, const float* __restrict__ w1,
@@ -816,6 +847,13 @@ static void launch_plan(dec_wedge_plan& P, const CoefSet<T>& c, const void* va, 
           if (vec) {
             k_w02v<<<grid2(m.nt / 4 + 1, kThreads, cnt), kThreads, 0, s>>>(m.nt, m.tv0.p, m.tv1.p, m.tv2.p, c.c[0].p,
                                                                              c.c[1].p, c.c[2].p, f, al, ob, sf, sl, so);
+            break;
+          }
+        }
+        if constexpr (sizeof(T) == 8) {
+          if (vec64) {
+            k_w02v64<<<grid2(m.nt / 2 + 1, kThreads, cnt), kThreads, 0, s>>>(m.nt, m.tv0.p, m.tv1.p, m.tv2.p, c.c[0].p,
+                                                                              c.c[1].p, c.c[2].p, f, al, ob, sf, sl, so);
             break;
           }
         }
