@@ -467,26 +467,36 @@ __device__ __forceinline__ __nv_bfloat16 bf16_part(float v, int k) {
   return __float2bfloat16_rn(r1 - __bfloat162float(mid));
 }
 
+// Everything a CTA needs before its first tile: the operands staged 16 bytes (one core row of 8 columns) a
+// thread, all in flight at once, the accumulator's TMEM, the mbarriers.  Only W1 and W2 are memory another
+// kernel may just have written; what needs no memory comes before the wait for the preceding kernel.  A launch
+// of few tiles is all setup: 8.3 us staged element by element, 7.1 in this form, 5.3 with its tiles dealt out
+// over the SMs (81,920 samples: 9.0 -> 6.5; icosphere L5 of 32 columns 15.5 -> 13.3; L7 129 -> 129).
 __device__ void tc_setup(TcSmem& sm, const MlpWeights& w) {
-  char* w1 = reinterpret_cast<char*>(sm.w1);
-  char* w2 = reinterpret_cast<char*>(sm.w2);
-  char* ones = reinterpret_cast<char*>(sm.ones);
-  char* bb1 = reinterpret_cast<char*>(sm.bb1);
-  char* bb2 = reinterpret_cast<char*>(sm.bb2);
-  for (int i = threadIdx.x; i < kTcRows * kMlpIn; i += blockDim.x)
-    *reinterpret_cast<__nv_bfloat16*>(ones + kmaj(i / kMlpIn, i % kMlpIn, kMlpIn)) =
-        __float2bfloat16_rn(i % kMlpIn < 3 ? 1.f : 0.f);
-  for (int i = threadIdx.x; i < kMlpH * kMlpIn; i += blockDim.x) {
-    const int j = i / kMlpIn, k = i % kMlpIn;
-    *reinterpret_cast<__nv_bfloat16*>(bb1 + kmaj(j, k, kMlpIn)) =
-        k < 3 ? bf16_part(w.hs.b1[j], k) : __float2bfloat16_rn(0.f);
-    *reinterpret_cast<__nv_bfloat16*>(bb2 + kmaj(j, k, kMlpIn)) =
-        k < 3 ? bf16_part(w.hs.b2[j], k) : __float2bfloat16_rn(0.f);
+  static_assert(kTcThreads >= kMlpH * kMlpH / 8 + kMlpH * kMlpIn / 8 + 3 * 128, "one pass of the setup");
+  const int t = threadIdx.x;
+  constexpr int n2 = kMlpH * kMlpH / 8, n1 = kMlpH * kMlpIn / 8;
+  auto put = [](void* base, int r, int k, int K, const uint4& v) {
+    *reinterpret_cast<uint4*>(reinterpret_cast<char*>(base) + kmaj(r, k, K)) = v;
+  };
+  auto pair = [](__nv_bfloat16 a, __nv_bfloat16 b) {
+    return (uint32_t)__bfloat16_as_ushort(a) | (uint32_t)__bfloat16_as_ushort(b) << 16;
+  };
+  if (t >= n2 + n1) {  // ones, bb1, bb2: columns 0..2, the rest zero
+    const int q = t - n2 - n1, which = q / 128, j = q % 128;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    if (which == 0) {
+      const __nv_bfloat16 one = __float2bfloat16_rn(1.f);
+      put(sm.ones, j, 0, kMlpIn, make_uint4(pair(one, one), (uint32_t)__bfloat16_as_ushort(one), 0, 0));
+      put(sm.ones, j, 8, kMlpIn, zero);
+    } else if (which < 3 && j < kMlpH) {
+      const float v = which == 1 ? w.hs.b1[j] : w.hs.b2[j];
+      void* bb = which == 1 ? sm.bb1 : sm.bb2;
+      put(bb, j, 0, kMlpIn,
+          make_uint4(pair(bf16_part(v, 0), bf16_part(v, 1)), (uint32_t)__bfloat16_as_ushort(bf16_part(v, 2)), 0, 0));
+      put(bb, j, 8, kMlpIn, zero);
+    }
   }
-  for (int i = threadIdx.x; i < kMlpH * kMlpIn; i += blockDim.x)
-    *reinterpret_cast<__nv_bfloat16*>(w1 + kmaj(i / kMlpIn, i % kMlpIn, kMlpIn)) = w.w1[i];
-  for (int i = threadIdx.x; i < kMlpH * kMlpH; i += blockDim.x)
-    *reinterpret_cast<__nv_bfloat16*>(w2 + kmaj(i / kMlpH, i % kMlpH, kMlpH)) = w.w2[i];
   if (threadIdx.x == 0) {
     for (int g = 0; g < kTcGroups; ++g)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.mbar[g])) : "memory");
@@ -497,6 +507,9 @@ __device__ void tc_setup(TcSmem& sm, const MlpWeights& w) {
                  "r"(kTcCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (t < n2) put(sm.w2, t / (kMlpH / 8), t % (kMlpH / 8) * 8, kMlpH, reinterpret_cast<const uint4*>(w.w2)[t]);
+  else if (t < n2 + n1) put(sm.w1, (t - n2) / 2, (t - n2) % 2 * 8, kMlpIn, reinterpret_cast<const uint4*>(w.w1)[t - n2]);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -635,7 +648,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_eval_tcg(int64_t n, const
   const int g = threadIdx.x / kTcRows, rr = threadIdx.x % kTcRows;
   uint32_t phase = 0;
   const int64_t ntiles = (n + kTcRows - 1) / kTcRows;
-  for (int64_t tile = (int64_t)blockIdx.x * kTcGroups + g; tile < ntiles; tile += (int64_t)gridDim.x * kTcGroups) {
+  for (int64_t tile = (int64_t)g * gridDim.x + blockIdx.x; tile < ntiles; tile += (int64_t)gridDim.x * kTcGroups) {
     const int64_t q = tile * kTcRows + rr;
     float f[16];
     if (q < n) {
@@ -682,7 +695,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_smooth_tcg(MlpWeights w, 
   // tile instead of a 64-bit one
   const uint32_t tiles_per_panel = (uint32_t)((nq + kTcRows - 1) / kTcRows);
   const uint32_t ntiles = tiles_per_panel * (uint32_t)np;
-  for (uint32_t tile = blockIdx.x * kTcGroups + g; tile < ntiles; tile += gridDim.x * kTcGroups) {
+  // a full round gives a CTA eight neighbouring tiles (shared neighbours' rows stay in its L1); the last one
+  // deals its tiles out over all the CTAs
+  const uint32_t round = gridDim.x * kTcGroups, full = ntiles / round * round;
+  const uint32_t last = full + g * gridDim.x + blockIdx.x;
+  uint32_t next;
+  for (uint32_t tile = full ? blockIdx.x * kTcGroups + g : last; tile < ntiles; tile = next) {
+    next = tile + round < full ? tile + round : tile < full ? last : ntiles;
     const uint32_t panel = tile / tiles_per_panel;
     const size_t po = (size_t)panel * pstride;
     const int64_t q = (int64_t)(tile - panel * tiles_per_panel) * kTcRows + rr;
@@ -740,9 +759,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_smooth_tcg(MlpWeights w, 
   tc_teardown(sm);
 }
 
-static unsigned tc_grid(long long tiles) {
-  const long long ctas = (tiles + kTcGroups - 1) / kTcGroups;
-  return (unsigned)std::max<long long>(1, std::min<long long>(ctas, (long long)num_sms()));
+static unsigned tc_grid(long long tiles) { return (unsigned)std::max<long long>(1, std::min<long long>(tiles, num_sms())); }
+
+// A launch that may start while the kernel before it drains; tc_setup waits for that one.
+template <class... KArgs, class... Args>
+static void tc_launch(void (*kernel)(KArgs...), long long tiles, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = tc_grid(tiles);
+  cfg.blockDim = kTcThreads;
+  cfg.dynamicSmemBytes = kTcSmemBytes;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  DEC_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
 }
 
 // The tcgen05 kernels' shared memory exceeds 48 KB, which needs each kernel's opt-in.
@@ -757,8 +789,7 @@ void launch_mlp_smooth(const MlpWeights& w, int n, int W, const int32_t* col, co
   if (w.engine == 1) {
     const long long tiles = ((long long)n * K + kTcRows - 1) / kTcRows * np;
     require(tiles < (1LL << 31), "mlp: too many sample tiles for one launch");
-    k_mlp_smooth_tcg<T, K><<<tc_grid(tiles), kTcThreads, kTcSmemBytes, s>>>(w, n, W, col, tab, diag, r, x, zero_x,
-                                                                          out, (size_t)n * K, np, w.err);
+    tc_launch(k_mlp_smooth_tcg<T, K>, tiles, s, w, n, W, col, tab, diag, r, x, zero_x, out, (size_t)n * K, np, w.err);
     DEC_CHECK_LAUNCH();
     return;
   }
