@@ -1059,48 +1059,76 @@ __global__ void __launch_bounds__(TB) k_coarse_eig2(int n, const double* __restr
 }
 
 // Column-major RHS block (nrhs vectors of length n, reference vertex order) <-> panels of K in the
-// level's internal order (iperm: reference -> internal).  A CTA moves a tile of kTile vertices x K
+// level's internal order (iperm: reference -> internal).  A CTA moves a tile of panel_tile(K) vertices x K
 // right-hand sides of one panel through shared memory, so both sides move in whole runs: a panel
-// row's K contiguous values, and kTile contiguous values of a vector.  (Element by element, one of
+// row's K contiguous values, and a tile's contiguous values of a vector.  (Element by element, one of
 // the two sides was a scattered 8-byte access: 1.7 / 3.3 TB/s at L8 x 32.)  Padding right-hand
 // sides (j >= nrhs) of the last panel are zero.
-constexpr int kTile = 32;
+//
+// Bound by memory: every thread has all its tile's values in flight, and a tile fills the CTA whatever K is
+// (512 values for K <= 8, 32 vertices above).  icosphere L8 x 32 to panels 87 -> 71 us, back 69 -> 73 (64
+// vertices a tile: 76 and 84; streaming hints: 74 and 71, but L8 x 16 39 and 40 against 34 and 35); L7 x 1
+// 5.3 -> 2.5 and 5.6 -> 2.5; L7 x 5 8.3 -> 5.5 and 8.1 -> 5.4.
+constexpr int kMoveThreads = 256;
+constexpr int panel_tile(int K) { return K >= 16 ? 32 : 512 / K; }
 
 template <int K>
-__global__ void __launch_bounds__(256) k_vectors_to_panels(int n, int nrhs, const int32_t* __restrict__ iperm,
-                                                           const double* __restrict__ src, double* __restrict__ dst) {
-  __shared__ double t[kTile][K + 1];
+__global__ void __launch_bounds__(kMoveThreads) k_vectors_to_panels(int n, int nrhs, const int32_t* __restrict__ iperm,
+                                                                    const double* __restrict__ src,
+                                                                    double* __restrict__ dst) {
+  constexpr int TL = panel_tile(K), E = TL * K / kMoveThreads;
+  __shared__ double t[TL][K + 1];
   const int p = blockIdx.y;
   double* dp = dst + (size_t)p * n * K;
-  for (int v0 = blockIdx.x * kTile; v0 < n; v0 += gridDim.x * kTile) {
-    for (int e = threadIdx.x; e < kTile * K; e += blockDim.x) {
-      const int k = e / kTile, dv = e % kTile, v = v0 + dv, j = p * K + k;
-      t[dv][k] = (v < n && j < nrhs) ? src[(size_t)j * n + v] : 0.0;
+  for (int v0 = blockIdx.x * TL; v0 < n; v0 += gridDim.x * TL) {
+    double x[E];
+    int row[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int e = threadIdx.x + i * kMoveThreads, v = v0 + e % TL, j = p * K + e / TL, w = v0 + e / K;
+      x[i] = (v < n && j < nrhs) ? src[(size_t)j * n + v] : 0.0;
+      row[i] = w < n ? iperm[w] : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int e = threadIdx.x + i * kMoveThreads;
+      t[e % TL][e / TL] = x[i];
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < kTile * K; e += blockDim.x) {
-      const int dv = e / K, k = e % K, v = v0 + dv;
-      if (v < n) dp[(size_t)iperm[v] * K + k] = t[dv][k];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int e = threadIdx.x + i * kMoveThreads;
+      if (row[i] >= 0) dp[(size_t)row[i] * K + e % K] = t[e / K][e % K];
     }
     __syncthreads();
   }
 }
 
 template <int K>
-__global__ void __launch_bounds__(256) k_panels_to_vectors(int n, int nrhs, const int32_t* __restrict__ iperm,
-                                                           const double* __restrict__ src, double* __restrict__ dst) {
-  __shared__ double t[kTile][K + 1];
+__global__ void __launch_bounds__(kMoveThreads) k_panels_to_vectors(int n, int nrhs, const int32_t* __restrict__ iperm,
+                                                                    const double* __restrict__ src,
+                                                                    double* __restrict__ dst) {
+  constexpr int TL = panel_tile(K), E = TL * K / kMoveThreads;
+  __shared__ double t[TL][K + 1];
   const int p = blockIdx.y;
   const double* sp = src + (size_t)p * n * K;
-  for (int v0 = blockIdx.x * kTile; v0 < n; v0 += gridDim.x * kTile) {
-    for (int e = threadIdx.x; e < kTile * K; e += blockDim.x) {
-      const int dv = e / K, k = e % K, v = v0 + dv;
-      if (v < n) t[dv][k] = sp[(size_t)iperm[v] * K + k];
+  for (int v0 = blockIdx.x * TL; v0 < n; v0 += gridDim.x * TL) {
+    double x[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int e = threadIdx.x + i * kMoveThreads, v = v0 + e / K;
+      x[i] = v < n ? sp[(size_t)iperm[v] * K + e % K] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int e = threadIdx.x + i * kMoveThreads;
+      t[e / K][e % K] = x[i];
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < kTile * K; e += blockDim.x) {
-      const int k = e / kTile, dv = e % kTile, v = v0 + dv, j = p * K + k;
-      if (v < n && j < nrhs) dst[(size_t)j * n + v] = t[dv][k];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int e = threadIdx.x + i * kMoveThreads, v = v0 + e % TL, j = p * K + e / TL;
+      if (v < n && j < nrhs) dst[(size_t)j * n + v] = t[e % TL][e / TL];
     }
     __syncthreads();
   }
@@ -1109,10 +1137,10 @@ __global__ void __launch_bounds__(256) k_panels_to_vectors(int n, int nrhs, cons
 // src (nrhs x n, reference order) -> dst panels; iperm: reference -> internal row.
 static void to_panels(int n, int nrhs, int K, int np, const int32_t* iperm, const double* src, double* dst,
                       cudaStream_t s) {
-  const dim3 g(grid_for(n, kTile, 16), np);
+  const dim3 g(grid_for(n, panel_tile(K), 16), np);
   switch (K) {
 #define DEC_K(KK) \
-  case KK: k_vectors_to_panels<KK><<<g, 256, 0, s>>>(n, nrhs, iperm, src, dst); break;
+  case KK: k_vectors_to_panels<KK><<<g, kMoveThreads, 0, s>>>(n, nrhs, iperm, src, dst); break;
     DEC_K(1) DEC_K(2) DEC_K(4) DEC_K(8) DEC_K(16) DEC_K(32)
 #undef DEC_K
     default: throw Error(DEC_ERR_INVALID_ARG, "multigrid: bad panel width");
@@ -1122,10 +1150,10 @@ static void to_panels(int n, int nrhs, int K, int np, const int32_t* iperm, cons
 // panels -> dst (nrhs x n, reference order).
 static void from_panels(int n, int nrhs, int K, int np, const int32_t* iperm, const double* src, double* dst,
                         cudaStream_t s) {
-  const dim3 g(grid_for(n, kTile, 16), np);
+  const dim3 g(grid_for(n, panel_tile(K), 16), np);
   switch (K) {
 #define DEC_K(KK) \
-  case KK: k_panels_to_vectors<KK><<<g, 256, 0, s>>>(n, nrhs, iperm, src, dst); break;
+  case KK: k_panels_to_vectors<KK><<<g, kMoveThreads, 0, s>>>(n, nrhs, iperm, src, dst); break;
     DEC_K(1) DEC_K(2) DEC_K(4) DEC_K(8) DEC_K(16) DEC_K(32)
 #undef DEC_K
     default: throw Error(DEC_ERR_INVALID_ARG, "multigrid: bad panel width");
@@ -1323,15 +1351,25 @@ __global__ void __launch_bounds__(256) k_ir_check(cudaGraphConditionalHandle h, 
   }
 }
 
-// Per-block partial sums of x² per right-hand side over the panels (same layout as k_residual64).
+// Per-block partial sums of x² per right-hand side over the panels (same layout as k_residual64).  Bound by
+// memory; four rows in flight a thread, added in order (as k_first_rhs: L8 x 32 57 -> 44 us).
 template <int K>
 __global__ void __launch_bounds__(TB) k_panel_sumsq(int n, const double* __restrict__ x, double* __restrict__ partial,
                                                     size_t pstride) {
   const int k = threadIdx.x % K;
   const size_t po = (size_t)blockIdx.y * pstride;
   double ss = 0.0;
-  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
-    double v = x[po + (size_t)i * K + k];
+  const int step = gridDim.x * (TB / K);
+  int i = blockIdx.x * (TB / K) + threadIdx.x / K;
+  for (; i < n - 3 * step; i += 4 * step) {  // four rows in flight, added in order
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = x[po + (size_t)(i + q * step) * K + k];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ss += v[q] * v[q];
+  }
+  for (; i < n; i += step) {
+    const double v = x[po + (size_t)i * K + k];
     ss += v * v;
   }
   __shared__ double sh[TB];
@@ -1353,7 +1391,19 @@ __global__ void __launch_bounds__(TB) k_first_rhs(int n, const double* __restric
   const int k = threadIdx.x % K;
   const size_t po = (size_t)blockIdx.y * pstride;
   double ss = 0.0;
-  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
+  const int step = gridDim.x * (TB / K);
+  int i = blockIdx.x * (TB / K) + threadIdx.x / K;
+  for (; i < n - 3 * step; i += 4 * step) {  // four rows in flight, added in order
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = x[po + (size_t)(i + q * step) * K + k];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      r[po + (size_t)(i + q * step) * K + k] = (T)v[q];
+      ss += v[q] * v[q];
+    }
+  }
+  for (; i < n; i += step) {
     const size_t ik = po + (size_t)i * K + k;
     const double v = x[ik];
     r[ik] = (T)v;
