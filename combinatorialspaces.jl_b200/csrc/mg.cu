@@ -988,36 +988,69 @@ __global__ void __launch_bounds__(TB) k_transfer(int rows, int W, const int32_t*
   }
 }
 
-// Coarsest level: x = A⁻¹ b with the dense FP64 inverse.  One CTA per (row, panel): its TB threads
-// are S = TB / K segments of the row's dot product for the K right-hand sides (segment g takes
-// columns g, g + S, g + 2S, ... into two FP64 sums), and the segments' sums meet in a fixed-order
-// tree in shared memory.  A thread per (row, right-hand side) running the whole row left a
-// 162-vertex level's solve latency-bound at 21 CTAs.
+// R rows of a dense coarsest-level product by a CTA: its TB threads are S = TB / K segments of the rows' dot
+// products for the K right-hand sides (segment g takes columns g, g + S, g + 2S, ... into two FP64 sums), and
+// the segments' sums meet in a fixed-order tree in shared memory (sh[r][k] at the end).  A thread per (row,
+// right-hand side) running the whole row left a 162-vertex level's solve latency-bound at 21 CTAs.  What is
+// left is latency, so a thread's next ten columns are loaded together: 162 vertices x 32 right-hand sides 6.7 us
+// a launch two columns at a time, 5.2 so, bit for bit (eight: 6.1; x 16: 4.1, 3.5).
+template <class T, int K, int R>
+__device__ __forceinline__ void coarse_rows(int n, const double* __restrict__ a, int rows, const T* __restrict__ bb,
+                                            double (&sh)[R][TB]) {
+  constexpr int S = TB / K, U = R == 1 ? 10 : 4;
+  const int k = threadIdx.x % K, g = threadIdx.x / K;
+  double s0[R], s1[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) s0[r] = s1[r] = 0.0;
+  int j = g;
+  for (; j + (U - 1) * S < n; j += U * S) {
+    double av[R][U];
+    T bv[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      bv[q] = bb[(size_t)(j + q * S) * K + k];
+#pragma unroll
+      for (int r = 0; r < R; ++r) av[r][q] = a[(size_t)min(r, rows - 1) * n + j + q * S];
+    }
+#pragma unroll
+    for (int q = 0; q < U; q += 2)
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        s0[r] += av[r][q] * to_d(bv[q]);
+        s1[r] += av[r][q + 1] * to_d(bv[q + 1]);
+      }
+  }
+  for (; j < n; j += 2 * S) {
+    const double b0 = to_d(bb[(size_t)j * K + k]), b1 = j + S < n ? to_d(bb[(size_t)(j + S) * K + k]) : 0.0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const double* ar = a + (size_t)min(r, rows - 1) * n;
+      s0[r] += ar[j] * b0;
+      if (j + S < n) s1[r] += ar[j + S] * b1;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) sh[r][threadIdx.x] = s0[r] + s1[r];
+  __syncthreads();
+  for (int st = S / 2; st > 0; st >>= 1) {
+    if (g < st)
+#pragma unroll
+      for (int r = 0; r < R; ++r) sh[r][threadIdx.x] += sh[r][threadIdx.x + st * K];
+    __syncthreads();
+  }
+}
+
+// Coarsest level: x = A⁻¹ b with the dense FP64 inverse, one CTA per (row, panel).
 template <class T, int K>
 __global__ void __launch_bounds__(TB) k_coarse(int n, const double* __restrict__ ainv, const T* __restrict__ b,
                                                T* __restrict__ x, size_t pstride) {
-  constexpr int S = TB / K;
   pdl_enter();
   const T* bb = b + (size_t)blockIdx.y * pstride;
   T* xx = x + (size_t)blockIdx.y * pstride;
-  const int k = threadIdx.x % K, g = threadIdx.x / K;
-  __shared__ double sh[TB];
+  __shared__ double sh[1][TB];
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    const double* a = ainv + (size_t)i * n;
-    double s0 = 0.0, s1 = 0.0;
-    int j = g;
-    for (; j + S < n; j += 2 * S) {
-      s0 += a[j] * to_d(bb[(size_t)j * K + k]);
-      s1 += a[j + S] * to_d(bb[(size_t)(j + S) * K + k]);
-    }
-    if (j < n) s0 += a[j] * to_d(bb[(size_t)j * K + k]);
-    sh[threadIdx.x] = s0 + s1;
-    __syncthreads();
-    for (int st = S / 2; st > 0; st >>= 1) {
-      if (g < st) sh[threadIdx.x] += sh[threadIdx.x + st * K];
-      __syncthreads();
-    }
-    if (g == 0) xx[(size_t)i * K + k] = from_d<T>(sh[k]);
+    coarse_rows<T, K, 1>(n, ainv + (size_t)i * n, 1, bb, sh);
+    if (threadIdx.x < K) xx[(size_t)i * K + threadIdx.x] = from_d<T>(sh[0][threadIdx.x]);
     __syncthreads();
   }
 }
@@ -1025,7 +1058,11 @@ __global__ void __launch_bounds__(TB) k_coarse(int n, const double* __restrict__
 // Coarsest-level solve for per-right-hand-side shifts c (coarse_solver 2): with
 // L = M⁻¹ K (M = ⋆0, K symmetric) and M^{1/2} L M^{-1/2} = Q Λ Qᵀ,
 // (L + c I)⁻¹ = E (Λ + c)⁻¹ F,  E = M^{-1/2} Q,  F = Qᵀ M^{1/2}.
-// Phase 1: y = (Λ + c)⁻¹ F b (FP64 scratch); phase 2: x = E y.
+// Phase 1: y = (Λ + c)⁻¹ F b (FP64 scratch); phase 2: x = E y.  Four rows a CTA: the eight groups of a batch
+// run these beside each other's sweeps, and a CTA per row took SM slots from those.  A batch of 64 solves over
+// eight meshes 2,360 -> 1,880 us, of 512 8,520 -> 8,375 (one row a CTA: 1,900 and 8,770; eight: 1,870 and 8,470;
+// a thread per row and right-hand side, as it was, 16 columns in flight: 2,330 and 8,455).
+constexpr int kEigRows = 4;
 template <class T, int K>
 __global__ void __launch_bounds__(TB) k_coarse_eig1(int n, const double* __restrict__ F, const double* __restrict__ lam,
                                                     const double* __restrict__ cs, const T* __restrict__ b,
@@ -1033,13 +1070,13 @@ __global__ void __launch_bounds__(TB) k_coarse_eig1(int n, const double* __restr
   pdl_enter();
   const T* bb = b + (size_t)blockIdx.y * pstride;
   double* yy = y + (size_t)blockIdx.y * pstride;
-  const int k = threadIdx.x % K;
-  const double c = cs[(size_t)blockIdx.y * K + k];
-  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
-    const double* a = F + (size_t)i * n;
-    double s = 0.0;
-    for (int j = 0; j < n; ++j) s += a[j] * to_d(bb[(size_t)j * K + k]);
-    yy[(size_t)i * K + k] = s / (lam[i] + c);
+  __shared__ double sh[kEigRows][TB];
+  for (int i = blockIdx.x * kEigRows; i < n; i += gridDim.x * kEigRows) {
+    const int rows = min(kEigRows, n - i);
+    coarse_rows<T, K, kEigRows>(n, F + (size_t)i * n, rows, bb, sh);
+    for (int e = threadIdx.x; e < rows * K; e += TB)
+      yy[(size_t)i * K + e] = sh[e / K][e % K] / (lam[i + e / K] + cs[(size_t)blockIdx.y * K + e % K]);
+    __syncthreads();
   }
 }
 
@@ -1049,12 +1086,12 @@ __global__ void __launch_bounds__(TB) k_coarse_eig2(int n, const double* __restr
   pdl_enter();
   const double* yy = y + (size_t)blockIdx.y * pstride;
   T* xx = x + (size_t)blockIdx.y * pstride;
-  const int k = threadIdx.x % K;
-  for (int i = blockIdx.x * (TB / K) + threadIdx.x / K; i < n; i += gridDim.x * (TB / K)) {
-    const double* a = E + (size_t)i * n;
-    double s = 0.0;
-    for (int j = 0; j < n; ++j) s += a[j] * yy[(size_t)j * K + k];
-    xx[(size_t)i * K + k] = from_d<T>(s);
+  __shared__ double sh[kEigRows][TB];
+  for (int i = blockIdx.x * kEigRows; i < n; i += gridDim.x * kEigRows) {
+    const int rows = min(kEigRows, n - i);
+    coarse_rows<double, K, kEigRows>(n, E + (size_t)i * n, rows, yy, sh);
+    for (int e = threadIdx.x; e < rows * K; e += TB) xx[(size_t)i * K + e] = from_d<T>(sh[e / K][e % K]);
+    __syncthreads();
   }
 }
 
@@ -3795,7 +3832,7 @@ static T* mu_cycle(const dec_mg& mg, Workspace& w, std::vector<LevelBufs<T>>& bu
     if (mg.opt.coarse_solver == 1)  // the smoother on the coarsest level (pre + post sweeps)
       return smooth<T, K>(mg, L, B, x, zero_x, std::max(1, mg.pre_at(l) + mg.post_at(l)), np, s);
     if (mg.opt.coarse_solver == 2) {  // per-RHS shifted solve through the eigendecomposition
-      const dim3 g(grid_for(L.n, TB / K, 64), np);
+      const dim3 g(grid_for(L.n, kEigRows, 8), np);
       add_bytes(2.0 * (double)L.n * L.n * 8.0 + (double)L.n * K * np * (2.0 * sizeof(T) + 16.0));
       launch_pdl(k_coarse_eig1<T, K>, g, dim3(TB), s, L.n, (const double*)mg.eigF.p, (const double*)mg.eigL.p,
                  (const double*)w.cs64.p, (const T*)B.b.p, w.ceig.p, (size_t)L.n * K);
