@@ -139,8 +139,9 @@ typedef enum dec_op_kind {
                                       ne x ne; the diagonal ⋆1 on planar circumcentric duals) */
   DEC_OP_INV_STAR1_GEOMETRIC = 15  /* dec_inv_hodge_star(1, sd, GeometricHodge()), FastDEC.jl:745-748,
                                       CUDA ext :93-96: y = (-⋆1)⁻¹ x by a Jacobi-preconditioned
-                                      BiCGSTAB solve in FP64 to 1e-14 relative residual (one host
-                                      read-back per reduction; not capturable in a CUDA graph) */,
+                                      BiCGSTAB solve in FP64 to 1e-14 relative residual (the loop
+                                      runs on the device, one host read-back per apply; not
+                                      capturable in a CUDA graph) */,
   DEC_OP_FLAT_SHARP = 16           /* ♭♯_mat(sd) (DiscreteExteriorCalculus.jl:1992; ♭ :687-714, ♯ :876-909):
                                       dual 1-form -> primal 1-form, ne x ne, <= 6 nnz per row (the
                                       matrix inside dec_wedge_product_pd/dp(1,1), FastDEC.jl:391-401) */,
@@ -427,10 +428,14 @@ dec_status dec_mg_solve_traffic(dec_mg* mg, int32_t nrhs, int32_t from_zero, int
 /* ---- the autotuner's table (no counterpart in the reference): the variant chosen per (kernel,
  *      dtype, shape, size bucket), process-wide, consulted when a kernel is launched or a solve graph
  *      captured.  Keys read "<kernel>/<dtype>/<shape>/n<floor(log2 size)>":
- *        ell/f32|f64/W7/n<rows>          rows per thread of the ELL apply (1, 2 or 4; 1 by default)
+ *        ell/f32|f64/W7/n<rows>          rows per thread of the ELL apply (1, 2 or 4; by default 1, and 2
+ *                                        for FP32 operators with two rows for each of the chip's threads)
  *        sweep/f32/K<width>/W<slots>/n<rows>  lanes per row of the FP32 smoothing sweep: the vector
  *                                        width 4 (default) or 2 (twice the lanes on a row)
- *      Every variant computes the same bits; only the time differs. ------------------------------ */
+ *        tail                            0: every level of a cycle by its own launches (by default the lower
+ *                                        levels run as one cluster kernel for up to 8 right-hand sides;
+ *                                        FP64 sums of its V(0,2) cycles may differ in the last bit)
+ *      Every other variant computes the same bits; only the time differs. ------------------------------ */
 /* Times each rows-per-thread variant of the operator's apply (operators stored as rows of 7 slots:
  * the Laplacian / Helmholtz operators of triangle meshes, a caller matrix of that width) on scratch
  * vectors, records the fastest in the table and returns it in *choice (0: the kernel has no variants). */
