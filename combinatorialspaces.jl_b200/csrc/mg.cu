@@ -244,18 +244,6 @@ __device__ __forceinline__ void l2_prefetch(const void* p, size_t bytes) {
   if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(e - a)));
 }
 
-// On unless DEC_B200_PDL=0.  Measured on B200 (same process, 10 L8 solves of 32 RHS; 20 L6
-// single-RHS FP64 solves): without the attribute 10,440 solves/s and 0.928 ms; with dependents
-// triggered at each kernel's start 10,250 and 0.891 ms (their blocks took SM slots from the large
-// finest-level kernels); with the implicit trigger at exit 10,525 and 0.840 ms.
-static bool pdl_enabled() {
-  static const bool on = [] {
-    const char* v = std::getenv("DEC_B200_PDL");
-    return !(v && v[0] == '0');
-  }();
-  return on;
-}
-
 template <class... KArgs, class... Args>
 static void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
