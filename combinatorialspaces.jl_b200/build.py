@@ -37,7 +37,7 @@ def nvcc() -> str:
 def _compile(src: str, force: bool) -> pathlib.Path:
     s = CSRC / src
     o = BUILD / (src + ".o")
-    deps = [s] + list(CSRC.glob("*.cuh")) + [INCLUDE / "dec_b200.h"]
+    deps = [s] + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + [INCLUDE / "dec_b200.h"]
     if not force and o.exists() and all(o.stat().st_mtime >= d.stat().st_mtime for d in deps):
         return o
     flags = list(COMMON)

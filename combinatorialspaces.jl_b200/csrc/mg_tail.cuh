@@ -23,57 +23,6 @@
 // 704 threads, 625 with 512, 615 with 384, 634 with 256 (852 without this kernel).
 #pragma once
 
-constexpr int kTailThreads = 384;
-constexpr int kTailLevels = 12;
-constexpr int kTailMaxCluster = 16;
-constexpr uint16_t kTailNone = 0xffff;     // a table's padding entry
-constexpr size_t kTailSmem = 224 * 1024;   // vectors and tables per CTA; the rest of the 227 KB is static
-
-enum TailType : uint8_t {
-  TT_RESTRICT_G, TT_LOAD, TT_LOADX, TT_STORE, TT_ADDU, TT_ZERO, TT_SWEEP, TT_AP, TT_RESTRICT, TT_PROLONG,
-  TT_COARSE, TT_CG  // from here on: phases that all threads of the CTA go through
-};
-// Buffers of a level.  Chebyshev / Jacobi: x, y (ping-pong, residual), b, d (correction form).
-// CG: x, r, b, two p's, q, Δx.
-enum TailBuf : uint8_t { TB_X = 0, TB_Y = 1, TB_B = 2, TB_D = 3, TB_P1 = 4, TB_Q = 5, TB_E = 6, TB_NBUF = 7 };
-// What a sweep does with its residual (SweepMode and sweep_rows' PV); none: a Chebyshev step.
-enum TailMode : uint8_t {
-  TM_RESID = 1,
-  TM_JACOBI = 2,
-  TM_FROM_ZERO = 4,  // x = 0
-  TM_PREV = 8,       // x_prev is what out holds (else 0)
-  TM_PZ = 16,        // x_prev = P z
-  TM_ADD = 32,       // out += the result
-  TM_OLD = TM_PREV | TM_ADD
-};
-
-// One phase, every table and vector as a byte offset in dynamic shared memory (resolved on the host: the
-// kernel reads five 16-byte words per phase instead of a level's descriptor).
-struct alignas(16) TailOp {
-  uint8_t type, mode, add, zero;     // mode: TailMode; add: prolong onto the iterate; zero: CG from x = 0
-  uint8_t barrier;                   // starts with a cluster barrier (else __syncthreads)
-  uint8_t split;                     // a dense product's rows / a restriction's rows are shared over the CTAs
-  uint8_t rep;                       // the level is kept by every CTA
-  uint8_t steps;                     // CG steps
-  int n, chunk;                      // rows of the phase, rows per CTA
-  uint32_t x, b, out, z;             // vectors: iterate / source, right-hand side, result, level + 1's
-  uint32_t t0, t1, t2, t3;           // col, off, diag, 1/diag | apc, apv, diag, 1/diag | rself, ridx, rw
-  uint32_t t4, t5;                   // parents pa, pb | CG: second p, q
-  uint16_t W, level;                 // slots per row; level of the hierarchy's tail (host only)
-  uint32_t t6;                       // CG: Δx
-  double p0, p1;                     // c1, c2 (1/θ for a first step, ω for Jacobi)
-};
-constexpr int kTailOpWords = sizeof(TailOp) / 16;
-static_assert(sizeof(TailOp) == 80, "five 16-byte words");
-
-// One level; the t_* are byte offsets of its tables in dynamic shared memory (the CTA's own rows, row-major).
-struct TailLevel {
-  int n, W, Wq, chunk;               // chunk: rows per CTA (n where every CTA keeps the level)
-  int rep, rchunk;                   // rep: kept by every CTA; rchunk: rows of level + 1 a CTA restricts
-  uint32_t t_col, t_off, t_diag, t_dinv, t_pa, t_pb, t_apc, t_apv, t_rself, t_ridx, t_rw;
-  uint32_t buf[TB_NBUF];             // byte offsets of the vectors
-};
-
 template <class T>
 struct TailPrm {
   const TailOp* ops;
