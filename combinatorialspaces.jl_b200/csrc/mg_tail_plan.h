@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <stdexcept>
 #include <vector>
 
 #include "dec_b200.h"
@@ -124,11 +125,16 @@ struct TailBuilder {
     op.t3 = L.t_dinv;
     op.t4 = L.t_pa;
     op.t5 = L.t_pb;
-    op.b = L.buf[TB_B];
+    op.b = buf(l, TB_B);
     ops.push_back(op);
     return ops.back();
   }
-  uint32_t buf(int l, int b) const { return cfg.lv[l - cfg.lt].buf[b]; }
+  // a vector's offset; one that the layout has not reserved would be the tables'
+  uint32_t buf(int l, int b) const {
+    const uint32_t o = cfg.lv[l - cfg.lt].buf[b];
+    if (o < cfg.image_bytes) throw std::logic_error("multigrid: a tail vector that its layout has not reserved");
+    return o;
+  }
   void interval(int l, double& theta, double& delta, double& sigma) const {
     const double hi = mg.lv[l].lmax, lo = hi / mg.opt.cheb_ratio;
     theta = (hi + lo) / 2;
@@ -402,11 +408,9 @@ bool tail_layout(const Mg& mg, TailPlan& c, size_t es, int K, int rep_rows) {
   }
   c.image_bytes = (uint32_t)at;
   for (int k = c.lt; k <= c.last; ++k) {
-    const int nb = cg ? TB_NBUF
-                   : (mg.opt.smoother == DEC_SMOOTH_CHEBYSHEV && mg.post_at(k) == 2 &&
-                      (mg.pre_at(k) > 0 || mg.opt.mu == 2 || k == 0))
-                       ? 4
-                       : 3;
+    // TB_D: a cycle entered with an iterate may end in the correction form (W-cycles, cycles after a first
+    // one, and on every level full multigrid, which prolongs before it cycles)
+    const int nb = cg ? TB_NBUF : mg.opt.smoother == DEC_SMOOTH_CHEBYSHEV && mg.post_at(k) == 2 ? 4 : 3;
     for (int b = 0; b < nb; ++b) c.lv[k - c.lt].buf[b] = take((size_t)c.lv[k - c.lt].chunk * es);
   }
   if (cg) {
