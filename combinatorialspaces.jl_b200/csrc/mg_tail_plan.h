@@ -324,9 +324,10 @@ struct TailBuilder {
   // Which phases start with a cluster barrier.  Rows of a split level are written by their CTA alone and
   // read by others through `gather`; a level that every CTA keeps is written by each, or pushed to all.
   // A phase needs the barrier when it reads what others may have written since the last one, writes what
-  // they may still read, follows a push, or pushes (the targets may still be read).
+  // they may still read, follows a push, or pushes (the targets may still be read).  The first access to
+  // another CTA's memory waits for all CTAs to run: a CG from zero reads none, but its sums store to all.
   void barriers() {
-    bool wrote = true, read = false, pushed = false;  // the first remote access waits for all CTAs to run
+    bool wrote = true, read = false, pushed = false, running = false;
     for (TailOp& op : ops) {
       const bool split = !cfg.lv[op.level].rep;
       const bool csplit = op.level + 1 < kTailLevels && cfg.lv[op.level + 1].n > 0 && !cfg.lv[op.level + 1].rep;
@@ -347,12 +348,14 @@ struct TailBuilder {
         case TT_CG: reads = split && !op.zero; writes = split; break;
         default: break;  // TT_STORE, TT_ADDU: the CTA's own rows
       }
-      op.barrier = ((reads && wrote) || (writes && read) || pushed || pushes) ? 1 : 0;
+      const bool sums = op.type == TT_CG && split;
+      op.barrier = ((reads && wrote) || (writes && read) || pushed || pushes || (sums && !running)) ? 1 : 0;
       if (op.barrier) wrote = read = pushed = false;
+      running |= op.barrier != 0;
       read |= reads;
       wrote |= writes;
       pushed |= pushes;
-      if (op.type == TT_CG && split) {  // its sums' barriers; x += Δx comes after the last
+      if (sums) {  // its sums' barriers; x += Δx comes after the last
         read = false;
         wrote = !op.zero;
       }

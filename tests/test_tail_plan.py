@@ -54,3 +54,13 @@ def test_stationary_programs(check, mesh, pre, post, K, npanels):
                 for coarse_solver in (0, 1):
                     on += check(HIERARCHIES[mesh], smoother, precision, pre, post, mu, inner, coarse_solver, K, npanels, cycles)[0] == "on"
     assert on > 0
+
+
+@pytest.mark.parametrize("mesh", HIERARCHIES)
+@pytest.mark.parametrize("pre,post", [(0, 2), (2, 0), (1, 2), (3, 3)])
+@pytest.mark.parametrize("K,npanels", [(1, 1), (2, 1), (8, 1), (4, 3)])
+def test_krylov_programs(check, mesh, pre, post, K, npanels):
+    on = 0
+    for mu, inner, cycles in ((1, 1, 1), (1, 3, 3), (2, 2, 0), (2, 1, 2)):
+        on += check(HIERARCHIES[mesh], CG, 0, pre, post, mu, inner, 0, K, npanels, cycles)[0] == "on"
+    assert on > 0
