@@ -1811,6 +1811,9 @@ struct Workspace {
   int K = 0, npanels = 0, prec = 0;
   TailCfg tail;
   std::map<int, TailProg> tprog;  // by tail_key(entry, parameter)
+  // tables and programs that a caller's own capture refers to: its graph stays replayable until the workspace goes
+  bool tail_captured = false;
+  std::vector<std::pair<TailCfg, std::map<int, TailProg>>> tail_kept;
   std::vector<LevelBufs<float>> f32;
   std::vector<LevelBufs<double>> f64;
   std::vector<LevelBufs<__half>> f16;  // precision 2: FP16 panels, FP32 arithmetic
@@ -1845,6 +1848,8 @@ struct Workspace {
       if (g) cudaGraphExecDestroy(g);
       g = nullptr;
     }
+    if (tail_captured) tail_kept.emplace_back(std::move(tail), std::move(tprog));
+    tail_captured = false;
     tprog.clear();  // they hold the sweep counts
     tail = TailCfg();
   }
@@ -4036,7 +4041,9 @@ void mg_full_multigrid(dec_mg* mg, double* u, const double* b, int nrhs, int cyc
   const int n = F.n;
   const size_t total = (size_t)n * w.K * w.npanels;
   // the tail's programs are built outside captures; a capture that meets a new `cycles` goes level by level
-  if (cycles < (1 << 16) && !stream_capturing(s)) {
+  if (stream_capturing(s)) {
+    w.tail_captured |= w.tail.on;
+  } else if (cycles < (1 << 16)) {
     ensure_tail(*mg, w);
     tail_program(*mg, w, TE_FMG, cycles);
   }

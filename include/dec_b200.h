@@ -288,7 +288,9 @@ dec_status dec_mg_level_op(const dec_mg* mg, int32_t level, const dec_op** out);
 dec_status dec_mg_cycles(dec_mg* mg, double* u, const double* b, int32_t nrhs, int32_t cycles, void* stream);
 /* full_multigrid(b, md, cycles, alg, μ) (Multigrid.jl:826-855): b restricted to the coarsest
  * level, then on the way up each level's solution is prolonged as the next level's initial guess
- * followed by `cycles` μ-cycles there; u (output) gets the finest level's result.  FP64. */
+ * followed by `cycles` μ-cycles there; u (output) gets the finest level's result.  FP64.  After a first
+ * call of the same nrhs it only enqueues kernels and can be captured in a caller's graph, which keeps the
+ * sweep counts of the capture. */
 dec_status dec_mg_full_multigrid(dec_mg* mg, double* u, const double* b, int32_t nrhs, int32_t cycles,
                                  void* stream);
 dec_status dec_mg_solve(dec_mg* mg, double* u, const double* b, int32_t nrhs, double rtol,
