@@ -1799,6 +1799,8 @@ struct LevelBufs {
 
 struct TailCfg : TailPlan {
   bool decided = false;
+  size_t fmg_phases = 0;          // of the full-multigrid programs built so far
+  int fmg_over = 1 << 16;         // a cycle count whose program would exceed kTailMaxPhases with them
   DArr<unsigned char> image;      // the tables, one image per CTA of a cluster
 };
 struct TailProg {
@@ -3241,7 +3243,15 @@ static void tail_program(dec_mg& mg, Workspace& w, int entry, int param) {
     else tail_pack<double>(mg, w.tail);
   }
   TailBuilder<dec_mg> b{mg, c, {}};
-  b.build(entry, param);
+  if (entry == TE_FMG) {
+    if (param >= c.fmg_over) return;
+    b.most = kTailMaxPhases - c.fmg_phases;
+  }
+  if (!b.build(entry, param)) {
+    if (entry == TE_FMG) w.tail.fmg_over = param;
+    return;
+  }
+  if (entry == TE_FMG) w.tail.fmg_phases += b.ops.size();
   TailProg p;
   p.ops.upload(b.ops);
   p.nops = (int)b.ops.size();
@@ -4043,7 +4053,7 @@ void mg_full_multigrid(dec_mg* mg, double* u, const double* b, int nrhs, int cyc
   // the tail's programs are built outside captures; a capture that meets a new `cycles` goes level by level
   if (stream_capturing(s)) {
     w.tail_captured |= w.tail.on;
-  } else if (cycles < (1 << 16)) {
+  } else {
     ensure_tail(*mg, w);
     tail_program(*mg, w, TE_FMG, cycles);
   }

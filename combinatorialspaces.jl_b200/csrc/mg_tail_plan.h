@@ -17,6 +17,9 @@ constexpr int kTailApW = 8;      // slots of a row of A P (kApW)
 constexpr int kTailThreads = 384;
 constexpr int kTailLevels = 12;
 constexpr int kTailMaxCluster = 16;
+// The most phases of a program (5 MB), and of all full-multigrid programs of a workspace together: cycle counts are
+// unrolled, and beyond this they go level by level.  Twelve levels of V(3,3) with 5 W-cycles a level have 15,100.
+constexpr size_t kTailMaxPhases = 1 << 16;
 constexpr uint16_t kTailNone = 0xffff;     // a table's padding entry
 constexpr size_t kTailSmem = 224 * 1024;   // vectors and tables per CTA; the rest of the 227 KB is static
 
@@ -108,6 +111,8 @@ struct TailBuilder {
   const Mg& mg;
   const TailPlan& cfg;
   std::vector<TailOp> ops;
+  size_t most = kTailMaxPhases;
+  bool full = false;  // more than `most` phases: the program is not usable
 
   bool cg() const { return mg.opt.smoother == DEC_SMOOTH_CG; }
   TailOp& emit(TailType t, int l) {
@@ -126,6 +131,8 @@ struct TailBuilder {
     op.t4 = L.t_pa;
     op.t5 = L.t_pb;
     op.b = buf(l, TB_B);
+    full = full || ops.size() >= most;
+    if (full && !ops.empty()) ops.pop_back();
     ops.push_back(op);
     return ops.back();
   }
@@ -223,6 +230,7 @@ struct TailBuilder {
   void residual(int l, int x, int out) { sweep(l, x, TB_B, out).mode = TM_RESID; }
   // the iterate of level l after one μ-cycle from buffer x (zero if zero_x)
   int cycle(int l, int x, bool zero_x, int mu) {
+    if (full) return x;
     if (cg()) {
       cg_smooth(l, zero_x, mg.pre_at(l));
       if (mg.pre_at(l) > 0) zero_x = false;
@@ -292,14 +300,15 @@ struct TailBuilder {
       prolong(l, z, zc, true);
       zero = false;
     }
-    for (int c = 0; c < cycles; ++c) {
+    for (int c = 0; c < cycles && !full; ++c) {
       z = cycle(l, z, zero, mg.opt.mu);
       zero = false;
     }
     if (zero) this->zero(l, z);
     return z;
   }
-  void build(int entry, int param) {
+  // false: too many phases
+  bool build(int entry, int param) {
     const int lt = cfg.lt;
     int z = TB_X;
     if (lt > 0) {
@@ -319,7 +328,8 @@ struct TailBuilder {
       z = fmg(lt, param);
     }
     emit(entry == TE_STEP && param ? TT_ADDU : TT_STORE, lt).x = buf(lt, z);
-    if (cfg.C > 1) barriers();
+    if (cfg.C > 1 && !full) barriers();
+    return !full;
   }
   // Which phases start with a cluster barrier.  Rows of a split level are written by their CTA alone and
   // read by others through `gather`; a level that every CTA keeps is written by each, or pushed to all.

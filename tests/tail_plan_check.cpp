@@ -4,8 +4,8 @@
 //
 // One hierarchy and entry per line of standard input:
 //   smoother precision pre post mu inner coarse_solver lc K npanels pfuse cycles levels (n W Wq ap_ok)*
-// finest level first; answers with "off", or "on <first level> <CTAs> <phases>", and a "fault ..." line for
-// each violation.
+// finest level first; answers with "off", or "on <first level> <CTAs> <phases>", "refused" behind it if a program
+// would be too long, and a "fault ..." line for each violation.
 #include <cstdio>
 #include <iostream>
 #include <map>
@@ -232,17 +232,22 @@ int main() {
       for (auto e : {std::pair<int, int>{TE_CYCLE, 0}, {TE_STEP, 0}, {TE_STEP, 1}}) entries.push_back(e);
     }
     size_t phases = 0;
+    bool refused = false;
     std::set<std::string> faults;
     for (auto& e : entries) {
       Checker ck{mg, plan, precision == 1 ? 4u : 8u, "entry " + std::to_string(e.first) + "/" + std::to_string(e.second), {}};
       ck.layout();
       TailBuilder<Hierarchy> b{mg, plan, {}};
-      b.build(e.first, e.second);
+      if (!b.build(e.first, e.second)) {
+        refused = true;
+        continue;
+      }
+      if (b.ops.size() > kTailMaxPhases) faults.insert("a program of more than kTailMaxPhases phases");
       phases += b.ops.size();
       for (unsigned seed = 1; seed <= (mg.opt.smoother == DEC_SMOOTH_CG ? 12u : 1u); ++seed) ck.run(b.ops, seed);
       faults.insert(ck.faults.begin(), ck.faults.end());
     }
-    std::printf("on %d %d %zu\n", plan.lt, plan.C, phases);
+    std::printf("on %d %d %zu%s\n", plan.lt, plan.C, phases, refused ? " refused" : "");
     for (auto& f : faults) std::printf("fault %s\n", f.c_str());
   }
 }

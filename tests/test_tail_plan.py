@@ -64,3 +64,13 @@ def test_krylov_programs(check, mesh, pre, post, K, npanels):
     for mu, inner, cycles in ((1, 1, 1), (1, 3, 3), (2, 2, 0), (2, 1, 2)):
         on += check(HIERARCHIES[mesh], CG, 0, pre, post, mu, inner, 0, K, npanels, cycles)[0] == "on"
     assert on > 0
+
+
+@pytest.mark.parametrize("smoother,mu", [(CHEBYSHEV, 1), (CG, 2)])
+def test_long_programs_are_refused(check, smoother, mu):
+    """Cycle counts are unrolled: a program is at most 65,536 phases (5 MB), whatever the count."""
+    for cycles, refused in ((5, False), (50, False), (20000, True), (65535, True)):
+        out = check(HIERARCHIES["sphere3"], smoother, cycles=cycles, mu=mu)
+        assert out[0] == "on" and ("refused" in out) == refused and int(out[3]) <= 65536
+    out = check(HIERARCHIES["sphere6"], smoother, mu=2, cycles=5)   # what dec_inverse_laplacian asks for by default
+    assert out[0] == "on" and "refused" not in out
