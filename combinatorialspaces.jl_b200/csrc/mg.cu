@@ -1812,10 +1812,10 @@ struct TailProg {
 struct Workspace {
   int K = 0, npanels = 0, prec = 0;
   TailCfg tail;
-  std::map<int, TailProg> tprog;  // by tail_key(entry, parameter)
+  std::map<int64_t, TailProg> tprog;  // by tail_key(entry, parameter)
   // tables and programs that a caller's own capture refers to: its graph stays replayable until the workspace goes
   bool tail_captured = false;
-  std::vector<std::pair<TailCfg, std::map<int, TailProg>>> tail_kept;
+  std::vector<std::pair<TailCfg, std::map<int64_t, TailProg>>> tail_kept;
   std::vector<LevelBufs<float>> f32;
   std::vector<LevelBufs<double>> f64;
   std::vector<LevelBufs<__half>> f16;  // precision 2: FP16 panels, FP32 arithmetic

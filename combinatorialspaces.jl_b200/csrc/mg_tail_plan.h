@@ -86,7 +86,7 @@ enum TailEntry {
   TE_FMG = 3,       // full multigrid with `parameter` cycles a level, b restricted from the level above (lt > 0)
                     // or loaded (lt = 0)
 };
-inline int tail_key(int entry, int param) { return entry << 16 | param; }
+inline int64_t tail_key(int entry, int param) { return (int64_t)entry << 32 | (uint32_t)param; }
 
 // Does the level's program use A P (k_sweep_ap's form of the first post-smoothing step)?
 template <class Mg>

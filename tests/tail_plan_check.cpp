@@ -231,6 +231,7 @@ int main() {
     } else {
       for (auto e : {std::pair<int, int>{TE_CYCLE, 0}, {TE_STEP, 0}, {TE_STEP, 1}}) entries.push_back(e);
     }
+    if (tail_key(TE_FMG, cycles) == tail_key(TE_FMG, cycles + (1 << 16))) std::puts("fault two cycle counts, one key");
     size_t phases = 0;
     bool refused = false;
     std::set<std::string> faults;
