@@ -833,7 +833,9 @@ struct KryPlan {
   unsigned blocks = 0;
   cudaGraphExec_t graph = nullptr;
   double* host = nullptr;  // pinned: true residual norm, ||b||
+  cudaEvent_t free = nullptr;  // after the epilogue that reads x: the next apply, on any stream, comes behind it
   ~KryPlan() {
+    if (free) cudaEventDestroy(free);
     if (graph) cudaGraphExecDestroy(graph);
     if (host) cudaFreeHost(host);
   }
@@ -848,6 +850,7 @@ static KryPlan* kry_plan(const dec_op& op) {
   plan->vec.alloc(11 * N + 3 * kKryMaxBlocks);
   plan->state.alloc(1);
   DEC_CUDA(cudaMemset(plan->state.p, 0, sizeof(KryState)));
+  DEC_CUDA(cudaEventCreateWithFlags(&plan->free, cudaEventDisableTiming));
   DEC_CUDA(cudaHostAlloc(&plan->host, 2 * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped));
   double* v = plan->vec.p;
   KryVecs& q = plan->q;
@@ -908,6 +911,7 @@ static void inverse_geometric_star(dec_op& op, const void* vx, void* vy, double 
   if (!op.kry) op.kry = kry_plan(op);
   const KryPlan& k = *op.kry;
   const size_t N = (size_t)n;
+  DEC_CUDA(cudaStreamWaitEvent(s, k.free, 0));
   if (op.dtype == DEC_F64) k_kry_init<<<k.blocks, kKryThreads, 0, s>>>(n, (const double*)vx, k.q, k.state.p);
   else k_kry_init<<<k.blocks, kKryThreads, 0, s>>>(n, (const float*)vx, k.q, k.state.p);
   DEC_CHECK_LAUNCH();
@@ -924,6 +928,7 @@ static void inverse_geometric_star(dec_op& op, const void* vx, void* vy, double 
   if (op.dtype == DEC_F64) k_epi<double><<<g, 256, 0, s>>>(N, k.q.x, (double*)vy, alpha, beta, beta != 0.0);
   else k_epi<float><<<g, 256, 0, s>>>(N, k.q.x, (float*)vy, alpha, beta, beta != 0.0);
   DEC_CHECK_LAUNCH();
+  DEC_CUDA(cudaEventRecord(k.free, s));
 }
 
 template <class T>
