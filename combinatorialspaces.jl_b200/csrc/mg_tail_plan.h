@@ -443,8 +443,12 @@ bool tail_layout(const Mg& mg, TailPlan& c, size_t es, int K, int rep_rows) {
 // L4: 435 / 288, 510 / 298; CG V-cycles on L6: 1,292 / 674, W-cycles 4,462 / 1,652.  A V(0,2)-cycle is
 // three phases a level: levels of more than kTailRowsFew rows per CTA stay outside (L6, FP32, 8 right-hand
 // sides: 391 / 378, with L5 inside 395 / 422), and few FP32 right-hand sides altogether (1: 292 / 301;
-// 4: 377 / 351).
+// 4: 377 / 351).  In FP32 over a dense coarsest level of more than kTailDenseFew vertices, V(0,2) stays outside
+// with more than 4 right-hand sides and W(0,2) with fewer than 4: a 65 x 65 grid over 9 x 9 V(0,2) 352 / 365 (8;
+// with 4 352 / 305), 257 x 257 over 9 x 9 W(0,2) 1,118 / 1,211 (1; 0.90 of it with 4), 129 x 97 over 17 x 13
+// 553 / 576 (1; 0.85 with 4); over 5 x 4 0.87 and 0.69 in their place, in FP64 between 0.99 and 1.01, and less.
 constexpr int kTailMinCluster = 8;
+constexpr int kTailDenseFew = 64;
 // K, npanels: the panels' width and count; prec: 0 FP64, 1 FP32; pfuse: the fused prolongation's mode;
 // held(C): how many clusters of C CTAs the device holds at a time.
 template <class Mg, class Held>
@@ -465,6 +469,9 @@ void tail_decide(const Mg& mg, TailPlan& c, int K, int npanels, int prec, int pf
   const int sweeps = mg.pre_at(c.last - 1) + mg.post_at(c.last - 1);
   const bool few = !cg && o.mu == 1 && sweeps <= 2;
   if (few && prec == 1 && groups < 4) return;
+  if (prec == 1 && o.coarse_solver == 0 && mg.pre_at(c.last - 1) == 0 && sweeps <= 2 && mg.lv[c.last].n > kTailDenseFew &&
+      (o.mu == 1 ? groups > 4 : groups < 4))
+    return;
   c.max_rows = few ? kTailRowsFew : kTailRows;
   auto fits = [&](int lt, int rep_rows) {
     c.lt = lt;

