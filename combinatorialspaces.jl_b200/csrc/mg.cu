@@ -1092,9 +1092,10 @@ __global__ void __launch_bounds__(TB) k_coarse_eig2(int n, const double* __restr
 // sides (j >= nrhs) of the last panel are zero.
 //
 // Bound by memory: every thread has all its tile's values in flight, and a tile fills the CTA whatever K is
-// (512 values for K <= 8, 32 vertices above).  icosphere L8 x 32 to panels 87 -> 71 us, back 69 -> 73 (64
-// vertices a tile: 76 and 84; streaming hints: 74 and 71, but L8 x 16 39 and 40 against 34 and 35); L7 x 1
-// 5.3 -> 2.5 and 5.6 -> 2.5; L7 x 5 8.3 -> 5.5 and 8.1 -> 5.4.
+// (512 values for K <= 8, 32 vertices above).  icosphere L8 x 32 to panels 87 -> 71 us (64 vertices a tile: 76;
+// streaming hints: 74, but L8 x 16 39 against 34); L8 x 16 52 -> 34 and back 46 -> 34; L7 x 1 5.3 -> 2.5 and
+// 5.6 -> 2.5; L7 x 5 8.3 -> 5.5 and 8.1 -> 5.4.  Panels of 32 go back by a plain loop: L8 x 32 70 us, 73 with the
+// values in flight, L7 x 32 17.7 and 16.8.
 constexpr int kMoveThreads = 256;
 constexpr int panel_tile(int K) { return K >= 16 ? 32 : 512 / K; }
 
@@ -1139,22 +1140,34 @@ __global__ void __launch_bounds__(kMoveThreads) k_panels_to_vectors(int n, int n
   const int p = blockIdx.y;
   const double* sp = src + (size_t)p * n * K;
   for (int v0 = blockIdx.x * TL; v0 < n; v0 += gridDim.x * TL) {
-    double x[E];
+    if constexpr (K == 32) {
+      for (int e = threadIdx.x; e < TL * K; e += blockDim.x) {
+        const int v = v0 + e / K;
+        if (v < n) t[e / K][e % K] = sp[(size_t)iperm[v] * K + e % K];
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < TL * K; e += blockDim.x) {
+        const int v = v0 + e % TL, j = p * K + e / TL;
+        if (v < n && j < nrhs) dst[(size_t)j * n + v] = t[e % TL][e / TL];
+      }
+    } else {
+      double x[E];
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int e = threadIdx.x + i * kMoveThreads, v = v0 + e / K;
-      x[i] = v < n ? sp[(size_t)iperm[v] * K + e % K] : 0.0;
-    }
+      for (int i = 0; i < E; ++i) {
+        const int e = threadIdx.x + i * kMoveThreads, v = v0 + e / K;
+        x[i] = v < n ? sp[(size_t)iperm[v] * K + e % K] : 0.0;
+      }
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int e = threadIdx.x + i * kMoveThreads;
-      t[e / K][e % K] = x[i];
-    }
-    __syncthreads();
+      for (int i = 0; i < E; ++i) {
+        const int e = threadIdx.x + i * kMoveThreads;
+        t[e / K][e % K] = x[i];
+      }
+      __syncthreads();
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int e = threadIdx.x + i * kMoveThreads, v = v0 + e % TL, j = p * K + e / TL;
-      if (v < n && j < nrhs) dst[(size_t)j * n + v] = t[e % TL][e / TL];
+      for (int i = 0; i < E; ++i) {
+        const int e = threadIdx.x + i * kMoveThreads, v = v0 + e % TL, j = p * K + e / TL;
+        if (v < n && j < nrhs) dst[(size_t)j * n + v] = t[e % TL][e / TL];
+      }
     }
     __syncthreads();
   }

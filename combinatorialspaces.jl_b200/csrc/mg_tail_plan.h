@@ -461,7 +461,7 @@ void tail_decide(const Mg& mg, TailPlan& c, int K, int npanels, int prec, int pf
   c.last = cg ? (int)mg.lv.size() - 1 : mg.lc;
   if (c.pfuse == 2 || c.last == 0) return;
   if (!cg && o.coarse_solver == 0 && mg.lv[c.last].n > kTailRepSmall) return;
-  if (cg && K > 8) return;  // blocks of fewer than 32 rows
+  if (cg && K > 8) return;  // the sums take blocks of 32 rows at least (a guard: 16 groups get no clusters of 8 here)
   const int groups = K * npanels;
   const size_t es = prec == 1 ? 4 : 8;
   for (c.C = kTailMaxCluster; c.C > 1 && held(c.C) < groups;) c.C /= 2;
