@@ -11,6 +11,7 @@
 #include <memory>
 #include <mutex>
 #include <type_traits>
+#include <vector>
 
 #include "mesh.cuh"
 #include "ops.cuh"
@@ -825,6 +826,43 @@ static void launch_ell(int n, int W, const int32_t* col, const T* val, const T* 
   else k_ell<T, 0><<<grid_for(n, kOpThreads), kOpThreads, 0, s>>>(n, W, col, val, x, y, a, b, hb);
 }
 
+// Two doubles that a kernel writes and the host reads: slots of one pinned page (256 at a time; memory of their
+// own beyond).  Pinning 16 bytes for each operator took 1 to 2.6 ms of its first apply, at times 100, and 0.4 ms to
+// give back; a copy to pageable memory instead 5 us of every apply.
+class HostSlots {
+ public:
+  static HostSlots& get() {
+    static HostSlots* slots = new HostSlots;  // outlives every operator
+    return *slots;
+  }
+  double* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!page_) {
+      DEC_CUDA(cudaHostAlloc(&page_, kSlots * 2 * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped));
+      for (int k = 0; k < kSlots; ++k) free_.push_back(page_ + 2 * k);
+    }
+    double* p = nullptr;
+    if (free_.empty()) {
+      DEC_CUDA(cudaHostAlloc(&p, 2 * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped));
+    } else {
+      p = free_.back();
+      free_.pop_back();
+    }
+    return p;
+  }
+  void give(double* p) {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (p >= page_ && p < page_ + 2 * kSlots) free_.push_back(p);
+    else cudaFreeHost(p);
+  }
+
+ private:
+  static constexpr int kSlots = 256;
+  std::mutex mu_;
+  double* page_ = nullptr;
+  std::vector<double*> free_;
+};
+
 // What the inverse geometric star keeps with its operator: the vectors, the state, the loop as a graph.
 struct KryPlan {
   DArr<double> vec;
@@ -837,7 +875,7 @@ struct KryPlan {
   ~KryPlan() {
     if (free) cudaEventDestroy(free);
     if (graph) cudaGraphExecDestroy(graph);
-    if (host) cudaFreeHost(host);
+    if (host) HostSlots::get().give(host);
   }
 };
 void kry_plan_delete(KryPlan* p) { delete p; }
@@ -851,7 +889,7 @@ static KryPlan* kry_plan(const dec_op& op) {
   plan->state.alloc(1);
   DEC_CUDA(cudaMemset(plan->state.p, 0, sizeof(KryState)));
   DEC_CUDA(cudaEventCreateWithFlags(&plan->free, cudaEventDisableTiming));
-  DEC_CUDA(cudaHostAlloc(&plan->host, 2 * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped));
+  plan->host = HostSlots::get().take();
   double* v = plan->vec.p;
   KryVecs& q = plan->q;
   for (double** d : {&q.b, &q.x, &q.r, &q.rh, &q.p[0], &q.p[1], &q.v[0], &q.v[1], &q.s, &q.t, &q.dinv}) {
