@@ -435,8 +435,10 @@ dec_status dec_mg_solve_traffic(dec_mg* mg, int32_t nrhs, int32_t from_zero, int
  *        sweep/f32/K<width>/W<slots>/n<rows>  lanes per row of the FP32 smoothing sweep: the vector
  *                                        width 4 (default) or 2 (twice the lanes on a row)
  *        tail                            0: every level of a cycle by its own launches (by default the lower
- *                                        levels run as one cluster kernel for up to 8 right-hand sides;
- *                                        FP64 sums of its V(0,2) cycles may differ in the last bit)
+ *                                        levels run as one kernel while every right-hand side, padding of the
+ *                                        panels included, gets a cluster of 8 CTAs: up to 8, or 12 as panels
+ *                                        of 4).  The kernel sums the dense coarsest product in another order
+ *                                        and rounds FP64 V(0,2) cycles otherwise: results differ in last bits
  *      Every other variant computes the same bits; only the time differs. ------------------------------ */
 /* Times each rows-per-thread variant of the operator's apply (operators stored as rows of 7 slots:
  * the Laplacian / Helmholtz operators of triangle meshes, a caller matrix of that width) on scratch
