@@ -30,7 +30,7 @@ struct Hierarchy {
   int post_at(int) const { return opt.post; }
 };
 
-struct Checker {
+struct Replay {
   const Hierarchy& mg;
   const TailPlan& c;
   size_t es;
@@ -236,7 +236,7 @@ int main() {
     bool refused = false;
     std::set<std::string> faults;
     for (auto& e : entries) {
-      Checker ck{mg, plan, precision == 1 ? 4u : 8u, "entry " + std::to_string(e.first) + "/" + std::to_string(e.second), {}};
+      Replay ck{mg, plan, precision == 1 ? 4u : 8u, "entry " + std::to_string(e.first) + "/" + std::to_string(e.second), {}};
       ck.layout();
       TailBuilder<Hierarchy> b{mg, plan, {}};
       if (!b.build(e.first, e.second)) {
